@@ -16,8 +16,8 @@
  * Per frame (a restatement in C is the oracle's wo_learned16_decode_batch):
  *   P[v]  = h(clamp(llr[v], -2048, 2048)), -0 made +0    (input staging)
  *   L_e   = h(P[v_e] - m_e)
- *   m1,m2 = the two smallest |L| of the row, each then min(., 2048)
- *   mu_e  = (|L_e| == m1) ? m2 : m1
+ *   mu_e  = min(2048, min over the other edges of |L|)   (min_others.cuh; with the
+ *           compare and select of two tracked minima 15% slower at r1/2 z=96)
  *   m'_e  = s_e * relu(h(a*mu_e - b))                    (one rounding: fma)
  *   P[v_e] = h(L_e + m'_e)
  * with h() rounding to binary16 and s_e the sign the other edges imply
@@ -32,7 +32,7 @@
  * Early exit per frame: after staging and after every iteration each frame's
  * syndrome is checked; a frame whose syndrome is zero is frozen and its
  * iteration count stops, while its partner decodes on. A frozen lane's
- * messages are set to +0 once and its row minima are masked to 0 in every
+ * messages are set to +0 once and its row minima are bounded by 0 in every
  * later layer, so its new messages are s * relu(a*0 - b) = +-0 (b >= 0) and
  * its posteriors are recomputed as (P - 0) + (+-0) = P exactly: they stay as
  * they were when the frame stopped, with no per-edge select. The CTA runs
@@ -53,6 +53,7 @@
 #include "codes.h"
 #include "device_util.cuh"
 #include "lms.cuh"
+#include "min_others.cuh"
 #include "nms_decode.cuh"
 
 namespace wldpc {
@@ -68,9 +69,11 @@ struct Lms16Args {
     int8_t* hard;           /* frames x n, 4-byte aligned */
     float* post;            /* frames x n or null, 16-byte aligned (may alias llr) */
     int32_t* status;        /* frames or null: iterations | synfail << 16 */
+    unsigned* err;
     long long frames;
     int iters;              /* iteration cap */
     int wrows;              /* trained iterations T; iteration t >= T uses row T-1 */
+    unsigned wait_limit_us = kWaitLimitUs;   /* bound of the staging waits */
     uint2 wab[kLmsMaxIter][kLmsMaxBlocks];   /* .x = (a, a), .y = (-b, -b) as f16x2 */
 };
 
@@ -104,30 +107,11 @@ __device__ __forceinline__ uint32_t h2_add(uint32_t a, uint32_t b)
     asm("add.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
     return d;
 }
-__device__ __forceinline__ uint32_t h2_min(uint32_t a, uint32_t b)
-{
-    uint32_t d;
-    asm("min.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
-    return d;
-}
-__device__ __forceinline__ uint32_t h2_max(uint32_t a, uint32_t b)
-{
-    uint32_t d;
-    asm("max.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
-    return d;
-}
 /* relu(a*b + c) with one rounding */
 __device__ __forceinline__ uint32_t h2_fma_relu(uint32_t a, uint32_t b, uint32_t c)
 {
     uint32_t d;
     asm("fma.rn.relu.f16x2 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
-    return d;
-}
-/* 0xffff in each lane where a == b, else 0 */
-__device__ __forceinline__ uint32_t h2_eq_mask(uint32_t a, uint32_t b)
-{
-    uint32_t d;
-    asm("set.eq.u32.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
     return d;
 }
 /* |a| per lane (an f16x2 abs, which the compiler can fold into the consuming
@@ -161,39 +145,6 @@ __device__ __forceinline__ uint32_t h2_stage(float x0, float x1)
     x0 = fminf(fmaxf(x0, -kLms16Clamp), kLms16Clamp);
     x1 = fminf(fmaxf(x1, -kLms16Clamp), kLms16Clamp);
     return h2_add(h2_from_floats(x0, x1), 0u);
-}
-
-/* m1 <= m2: per lane the two smallest of v[LO] .. v[HI-1] (non-negative
- * binary16 values, multiplicity counted), by a balanced tree of min/max;
- * equal to the sequential scan from +inf. */
-template <int LO, int HI, int D>
-__device__ __forceinline__ void two_min_h2(const uint32_t (&v)[D], uint32_t& m1, uint32_t& m2)
-{
-    static_assert(HI - LO >= 2, "two_min_h2 needs two values");
-    if constexpr (HI - LO == 2) {
-        m1 = h2_min(v[LO], v[LO + 1]);
-        m2 = h2_max(v[LO], v[LO + 1]);
-    } else if constexpr (HI - LO == 3) {
-        uint32_t a1, a2;
-        two_min_h2<LO, LO + 2>(v, a1, a2);
-        const uint32_t c = v[LO + 2];
-        m1 = h2_min(a1, c);
-        m2 = h2_min(h2_max(a1, c), a2);
-    } else {
-        constexpr int H = HI - LO;
-        constexpr int MID = LO + (H >= 16 ? 8 * (H / 16) : H >= 8 ? 4 * (H / 8) : 2 * (H / 4));
-        uint32_t a1, a2, b1, b2;
-        two_min_h2<LO, MID>(v, a1, a2);
-        if constexpr (HI - MID == 1) {
-            const uint32_t c = v[MID];
-            m1 = h2_min(a1, c);
-            m2 = h2_min(h2_max(a1, c), a2);
-        } else {
-            two_min_h2<MID, HI>(v, b1, b2);
-            m1 = h2_min(a1, b1);
-            m2 = h2_min(h2_max(a1, b1), h2_min(a2, b2));
-        }
-    }
 }
 
 template <int R, int Z>
@@ -329,18 +280,15 @@ lms16_decode_kernel(const __grid_constant__ Lms16Args a)
                     A[e] = h2_abs(L[e]);
                     sgn ^= L[e];
                 });
-                uint32_t m1, m2;
-                two_min_h2<0, d>(A, m1, m2);
-                m1 = h2_min(m1, kH2Clamp) & am;
-                m2 = h2_min(m2, kH2Clamp) & am;
+                uint32_t mu[d];
+                /* clamped at 2048; a frozen lane's bound is 0, so its minima are too */
+                min_others<MinH2, d, true>(A, mu, kH2Clamp & am);
                 /* positive LLR = bit 1: the extrinsic sign flips on odd-degree rows */
                 const uint32_t fb = (sgn ^ ((d & 1) ? kH2Sign : 0u)) & kH2Sign;
                 static_for<d>([&](auto E_) {
                     constexpr int e = decltype(E_)::value;
-                    const uint32_t eq = h2_eq_mask(A[e], m1);
-                    const uint32_t mu = (eq & m2) | (~eq & m1);
                     const uint2 ab = wab[b0 + e];
-                    const uint32_t mag = h2_fma_relu(ab.x, mu, ab.y);
+                    const uint32_t mag = h2_fma_relu(ab.x, mu[e], ab.y);
                     const uint32_t msg = mag | ((L[e] ^ fb) & kH2Sign);
                     Mr[b0 + e] = msg;
                     const uint32_t pn = h2_add(L[e], msg);
