@@ -9,6 +9,7 @@
 #include <cuda_runtime.h>
 #include "encode.cuh"
 #include "nms_decode.cuh"
+#include "unit_launch.cuh"
 
 namespace wldpc {
 
@@ -73,6 +74,7 @@ struct TdmpLaunch {
     int frames_per_cta;
     int smem;           /* dynamic shared memory bytes (run-time z: 96 z) */
     bool runtime_z;     /* z, shifts and columns are passed in DecodeArgs */
+    UnitLaunch<DecodeArgs> unit;   /* large batches, where it is the faster */
 };
 /* entry for (rate, z, mode) or null if not built */
 const TdmpLaunch* tdmp_entry(int rate, int z, int mode);

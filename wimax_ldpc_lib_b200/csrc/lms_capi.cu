@@ -273,6 +273,7 @@ static int lms16_launch_decode(wldpc_lms* h, const float* llr, int8_t* hard, flo
     a.hard = hard;
     a.post = post;
     a.status = status;
+    a.err = h->err;
     a.frames = (long long)frames;
     a.iters = h->cap;
     a.wrows = h->T;
@@ -280,6 +281,10 @@ static int lms16_launch_decode(wldpc_lms* h, const float* llr, int8_t* hard, flo
         for (int b = 0; b < h->nblk; b++)
             a.wab[t][b] = make_uint2(half_pair_bits(h->w.a[t][b]), half_pair_bits(-h->w.b[t][b]));
     const LmsLaunch* k = h->k;
+    if (unit_takes(k->unit16, a.frames)) {
+        CU(launch_unit(k->unit16, a, st));
+        return WLDPC_OK;
+    }
     const long long ctas = ((long long)frames + k->frames16 - 1) / k->frames16;
     k->decode16<<<(unsigned)ctas, k->threads16, 0, st>>>(a);
     CU(cudaGetLastError());
@@ -301,9 +306,15 @@ static int lms_launch_decode(wldpc_lms* h, const float* llr, int8_t* hard, float
     a.frames = (long long)frames;
     a.iters = h->cap;
     a.wrows = h->T;
-    for (int t = 0; t < h->T; t++)
-        for (int b = 0; b < h->nblk; b++) a.wab[t][b] = make_float2(h->w.a[t][b], h->w.b[t][b]);
     const LmsLaunch* k = h->k;
+    const bool unit = unit_takes(k->unit, a.frames);
+    const float scale = unit ? 0.5f : 1.0f;   /* the unit kernel takes half the weights (LearnedRow) */
+    for (int t = 0; t < h->T; t++)
+        for (int b = 0; b < h->nblk; b++) a.wab[t][b] = make_float2(h->w.a[t][b] * scale, h->w.b[t][b] * scale);
+    if (unit) {
+        CU(launch_unit(k->unit, a, st));
+        return WLDPC_OK;
+    }
     if (k->smem > 48 * 1024)
         CU(cudaFuncSetAttribute(k->decode, cudaFuncAttributeMaxDynamicSharedMemorySize, k->smem));
     const long long ctas = ((long long)frames + k->frames_per_cta - 1) / k->frames_per_cta;

@@ -4,6 +4,7 @@
 
 #include "lms.cuh"
 #include "lms16.cuh"
+#include "unit_decode.cuh"
 
 namespace wldpc {
 
@@ -19,6 +20,8 @@ struct LmsLaunch {
     int train_smem;          /* train CTA = z threads, one frame */
     void (*decode16)(const Lms16Args);   /* packed-half decoder (lms16.cuh) */
     int threads16, frames16;             /* its CTA size and frames per CTA (static shared memory) */
+    UnitLaunch<LmsArgs> unit;            /* large batches */
+    UnitLaunch<Lms16Args> unit16;
 };
 
 const LmsLaunch* lms_entry(int rate, int z);

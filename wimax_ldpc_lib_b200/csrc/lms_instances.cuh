@@ -1,8 +1,9 @@
 /* Instantiation unit of the learned min-sum kernels (lms.cuh, lms16.cuh) for
  * one code rate and one half of the 19 expansion factors. The Makefile
  * compiles it once per (rate, half) as CUDA with -DWLDPC_LMS_RATE=r and
- * -DWLDPC_LMS_HALF=h (h = 0: z = 24..56, h = 1: z = 60..96), so the 342
- * kernels (decoder, training and packed-binary16 decoder for 114 codes) build
+ * -DWLDPC_LMS_HALF=h (h = 0: z = 24..56, h = 1: z = 60..96), so the 570
+ * kernels (per code the decoder and the packed-binary16 decoder, each for small
+ * and for large batches, and the training kernel) build
  * in 12 parallel translation units. Each unit defines the dispatch rows
  * kLms_r<r>_h<h>[] that lms_entry() (lms_capi.cu) looks up. */
 #include "lms_dispatch.cuh"
@@ -17,7 +18,8 @@ namespace wldpc {
     {Z, &lms_decode_kernel<WLDPC_LMS_RATE, Z>, LmsShape<WLDPC_LMS_RATE, Z>::THREADS,                           \
      LmsShape<WLDPC_LMS_RATE, Z>::G, LmsShape<WLDPC_LMS_RATE, Z>::SMEM, &lms_train_kernel<WLDPC_LMS_RATE, Z>, \
      LmsTrainShape<WLDPC_LMS_RATE, Z>::SMEM, &lms16_decode_kernel<WLDPC_LMS_RATE, Z>,                         \
-     Lms16Shape<WLDPC_LMS_RATE, Z>::THREADS, Lms16Shape<WLDPC_LMS_RATE, Z>::FRAMES}
+     Lms16Shape<WLDPC_LMS_RATE, Z>::THREADS, Lms16Shape<WLDPC_LMS_RATE, Z>::FRAMES,                          \
+     unit_launch<WLDPC_LMS_RATE, Z, LearnedRow>(), unit_launch16<WLDPC_LMS_RATE, Z>()}
 
 #define WLDPC_LMS_PASTE2(a, b, c, d) a##b##c##d
 #define WLDPC_LMS_PASTE(a, b, c, d) WLDPC_LMS_PASTE2(a, b, c, d)

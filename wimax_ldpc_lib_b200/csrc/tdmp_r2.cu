@@ -1,11 +1,13 @@
 /* Normalized min-sum TDMP decoders for rate enum 2, specialised on each of
  * the 19 expansion factors (the shipped reference flavour, the hot path). */
 #include "codec_kernels.cuh"
+#include "unit_decode.cuh"
 
 namespace wldpc {
 
 #define WLDPC_TDMP_NMS(Z) \
-    {&tdmp_decode_kernel<2, Z, kNms>, TdmpShape<2, Z>::THREADS, TdmpShape<2, Z>::G, TdmpShape<2, Z>::SMEM, false}
+    {&tdmp_decode_kernel<2, Z, kNms>, TdmpShape<2, Z>::THREADS, TdmpShape<2, Z>::G, TdmpShape<2, Z>::SMEM, false, \
+     unit_launch<2, Z, PlainRow>()}
 
 extern const TdmpLaunch kTdmpNms_r2[kNumZ] = {
     WLDPC_TDMP_NMS(24), WLDPC_TDMP_NMS(28), WLDPC_TDMP_NMS(32), WLDPC_TDMP_NMS(36), WLDPC_TDMP_NMS(40),
