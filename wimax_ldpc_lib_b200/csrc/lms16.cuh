@@ -107,6 +107,19 @@ __device__ __forceinline__ uint32_t h2_add(uint32_t a, uint32_t b)
     asm("add.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
     return d;
 }
+__device__ __forceinline__ uint32_t h2_mul(uint32_t a, uint32_t b)
+{
+    uint32_t d;
+    asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+    return d;
+}
+/* a*b + c with one rounding */
+__device__ __forceinline__ uint32_t h2_fma(uint32_t a, uint32_t b, uint32_t c)
+{
+    uint32_t d;
+    asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
+    return d;
+}
 /* relu(a*b + c) with one rounding */
 __device__ __forceinline__ uint32_t h2_fma_relu(uint32_t a, uint32_t b, uint32_t c)
 {

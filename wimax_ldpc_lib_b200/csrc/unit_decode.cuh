@@ -24,14 +24,13 @@
  * decoders' units restart together, because their weights go by iteration
  * (one row for the whole unit).
  *
- * Measured against the one-frame-per-CTA kernels (ms, outputs identical):
- * r1/2 z=96, 65,536 frames: plain 2.18 -> 2.05, learned fp32 1.32 -> 1.33
- * alone on the SM's ALU pipe either way (1.16 at 262,144 frames against the
- * kernel with tracked minima), binary16 (131,072) 1.66 -> 1.50; r2/3B z=44,
- * 20,011 frames: 0.326 -> 0.261, 0.321 -> 0.193; r5/6 z=60, 30,011 frames:
- * learned 0.324 -> 0.256; r3/4B z=28, 30,001 frames: 0.255 -> 0.193,
- * 0.221 -> 0.140, binary16 0.193 -> 0.095. Now bound by the ALU and XU pipes
- * (plain: 77% and 67% busy, 70% of issue slots) and by issue (learned: 76%).
+ * Measured against the one-frame-per-CTA kernels of the same arithmetic (ms,
+ * outputs identical): r1/2 z=96, 65,536 frames: plain 2.18 -> 2.05, learned
+ * fp32 1.32 -> 1.29, binary16 (131,072) 1.66 -> 1.48; r2/3B z=44, 20,011
+ * frames: plain 0.326 -> 0.261, learned 0.26 -> 0.19; r3/4B z=28, 30,001
+ * frames: 0.255 -> 0.193, 0.19 -> 0.14, binary16 0.17 -> 0.095. What binds
+ * now: the ALU and XU pipes for plain (77% and 67% busy, 70% of the issue
+ * slots), issue for learned (79-82%), the ALU pipe for binary16 (68%).
  *
  * Every wait on a copy is bounded: when one expires the unit records
  * kErrWaitTimeout, waits (bounded) for the copies it has in flight and ends.
@@ -96,8 +95,9 @@ struct LearnedRow {
     static __device__ __forceinline__ int cap(const LmsArgs& a) { return a.iters; }
     __device__ __forceinline__ void iteration(const LmsArgs& a, int t)
     {
-        /* the shuffle tells the compiler that the row is the same in every lane */
-        w = a.wab[__shfl_sync(0xffffffffu, t < a.wrows ? t : a.wrows - 1, 0)];
+        /* a uniform row (by a shuffle from lane 0) turned the weights into uniform
+         * registers, of which an instruction takes one: 7% more instructions, 2.7% slower */
+        w = a.wab[t < a.wrows ? t : a.wrows - 1];
     }
     /* x: posteriors, m: old messages in, new ones out, pn: new posteriors.
      * loaded() is called once the old messages have been read. */
@@ -624,6 +624,7 @@ unit_decode16_kernel(const __grid_constant__ Lms16Args a)
             unit_clear_messages<R>(M, tm);
         }
         const bool busy = owner && ((act >> (2 * g)) & 3u);
+        /* the shuffle makes the row uniform: 1.5% faster here, unlike in LearnedRow */
         const uint2* const w = a.wab[__shfl_sync(0xffffffffu, t < a.wrows ? t : a.wrows - 1, 0)];
         uint32_t last_par = 0;
         static_for<MB>([&](auto I) {
@@ -648,12 +649,16 @@ unit_decode16_kernel(const __grid_constant__ Lms16Args a)
             });
             tm_ld<layer_degree(R, ni)>(M, tm + block_index(R, ni, 0));
             min_others<MinH2, d, true>(A, mu, kH2Clamp);
-            const uint32_t fb = (sgn ^ ((d & 1) ? kH2Sign : 0u)) & kH2Sign;
+            /* the sign as a factor +-1 (exact): the FMA pipe has room, the ALU pipe,
+             * 68% busy with the sign ORed in, has not (262,144 r1/2 z=96 frames 3.02 ->
+             * 2.96 ms); the posterior as one fma, L + msg exactly */
+            const uint32_t one = ((sgn ^ ((d & 1) ? kH2Sign : 0u)) & kH2Sign) | 0x3c003c00u;
             static_for<d>([&](auto E) {
                 const uint2 ab = w[b0 + E];
                 const uint32_t mag = h2_fma_relu(ab.x, mu[E], ab.y);
-                m[E] = mag | ((L[E] ^ fb) & kH2Sign);
-                const uint32_t pn = h2_add(L[E], m[E]);
+                const uint32_t sign = (L[E] & kH2Sign) ^ one;
+                m[E] = h2_mul(mag, sign);
+                const uint32_t pn = h2_fma(mag, sign, L[E]);
                 if ((FULL && G == 1) || busy) *ptr[E] = pn;
                 if constexpr (LAST) last_par ^= pn;
             });

@@ -17,9 +17,10 @@ enum UnitKind : int { kUnitPlain = 0, kUnitLearned = 1, kUnitLearned16 = 2 };
  * 2500, 5000 and 30,000 frames (outputs identical); a code's line is the first
  * of those sizes from which on the unit kernel was never more than 1% slower.
  * Digits: 1: 64 frames, 2: 600, 3: 2500, 4: 5000, 5: 20,000, 0: never.
- * At 30,000 frames the unit kernel took 0.46 to 1.0 of the other's time:
- * plain 0.65-0.99 (rate 5/6, degree 20, spills and keeps the other kernel at
- * most z), learned fp32 0.52-0.95, binary16 0.40-0.95. */
+ * At 30,000 frames the unit kernel took, where it is used, 0.64-0.99 of the
+ * other's time for plain (rate 5/6, degree 20, spills in 80 registers and
+ * keeps the other kernel at most z), 0.55-0.99 for learned fp32 and 0.47-0.99
+ * for binary16; least where z is no multiple of 16. */
 constexpr const char* kUnitMin[3][6] = {
     {
         "5153435111212141113",
@@ -30,20 +31,20 @@ constexpr const char* kUnitMin[3][6] = {
         "0000000004030100500",
     },
     {
-        "5221313111111131112",
-        "1111311111211131112",
-        "1111313311111131112",
-        "1113335111211331112",
-        "1111414111111121111",
-        "3353330333423241113",
+        "3151315111111151115",
+        "4153510111013351113",
+        "1113315311421331115",
+        "1113530111112331215",
+        "2111440111132231110",
+        "5154050344033342330",
     },
     {
-        "1123314111311131113",
-        "1131314111311131113",
-        "1141314111511131114",
-        "2143445332511131113",
-        "2123214111311131113",
-        "0405450333033343435",
+        "1153415111511151114",
+        "1143335111533331113",
+        "1154315331533343115",
+        "3154440333011343314",
+        "2153310131033331113",
+        "5515550554044454540",
     },
 };
 constexpr long long unit_min_frames(UnitKind kind, int rate, int z)
