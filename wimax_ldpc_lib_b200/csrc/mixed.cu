@@ -125,6 +125,7 @@ static MixedKernel mixed_kernel(int ti, int layout, int rows, int rate)
 
 struct wldpc_mixed {
     unsigned max_iter;
+    bool tuned = false;                    /* the caller chose (or autotuned): untuned_for() does not */
     int threads = 96, layout = kMsgRegisters, chunk = 16;
     int rows = 1;                          /* expanded rows per thread: z / rows threads per frame */
     int launch = WLDPC_MIXED_CONCURRENT;   /* the six rate grids: concurrent or one after another */
@@ -146,6 +147,21 @@ struct wldpc_mixed {
         bool operator==(const Key& o) const { return memcmp(this, &o, sizeof(Key)) == 0; }
     } key{};
 };
+
+/* Without a tuning of the caller's own: CTAs of 192 threads (twice the slots
+ * of 96, so less of a CTA waits at an item's end) and items that grow with the
+ * batch. A small batch needs short items, or a few CTAs work through long ones
+ * while the rest of the GPU is idle; a large one long items, which refill
+ * their slots more often and build the address table less often. Every chunk
+ * of 1 to 24 frames and both CTA sizes timed on batches of all 114 codes (ms,
+ * this choice against the 96 threads and 16 frames that it replaces): 256
+ * frames 0.10 / 0.25, 1024 0.16 / 0.54, 4096 0.37 / 1.16, 16,384 0.95 / 2.63,
+ * 65,536 3.06 / 5.44, 262,144 11.3 / 12.4. */
+static void untuned_for(wldpc_mixed* h, size_t frames)
+{
+    h->threads = 192;
+    h->chunk = frames <= 600 ? 1 : frames <= 12000 ? 2 : frames <= 45000 ? 4 : frames <= 150000 ? 8 : 16;
+}
 
 static int mixed_enqueue(wldpc_mixed* h, const uint8_t* variant, const long long* offset, const float* llr,
                          int8_t* hard, float* post, int32_t* status, size_t frames, cudaStream_t st)
@@ -310,6 +326,7 @@ int wldpc_mixed_set_tuning(wldpc_mixed* h, int threads, int layout, int chunk, i
     if (threads != 96 && threads != 192) return WLDPC_ERR_ARG;
     if (layout != WLDPC_MIXED_MSG_REGISTERS && layout != WLDPC_MIXED_MSG_SHARED) return WLDPC_ERR_ARG;
     if (launch != WLDPC_MIXED_CONCURRENT && launch != WLDPC_MIXED_SERIAL) return WLDPC_ERR_ARG;
+    h->tuned = true;
     h->threads = threads;
     h->layout = layout;
     h->chunk = chunk;
@@ -330,6 +347,7 @@ int wldpc_mixed_get_tuning(wldpc_mixed* h, int* threads, int* layout, int* chunk
 int wldpc_mixed_set_rows_per_thread(wldpc_mixed* h, int rows)
 {
     if (!h || (rows != 1 && rows != 2)) return WLDPC_ERR_ARG;
+    h->tuned = true;
     h->rows = rows;
     return WLDPC_OK;
 }
@@ -362,6 +380,7 @@ int wldpc_mixed_decode_device(wldpc_mixed* h, const uint8_t* variant, const int6
     if (frames == 0) return WLDPC_OK;
     if (frames > 0x7fffffff) return WLDPC_ERR_ARG;
     int rc;
+    if (!h->tuned) untuned_for(h, frames);
     const size_t max_items = kRates * (frames / (size_t)h->chunk + kNumZ + 1);
     if ((rc = h->rank.reserve(frames * sizeof(int))) || (rc = h->perm.reserve(frames * sizeof(int))) ||
         (rc = h->items.reserve(max_items * sizeof(MixedItem))))
@@ -429,6 +448,7 @@ int wldpc_mixed_autotune(wldpc_mixed* h, const uint8_t* variant, const int64_t* 
                          int8_t* decoded, size_t frames, int repeats, float* best_ms)
 {
     if (!h || repeats < 1) return WLDPC_ERR_ARG;
+    h->tuned = true;
     static const int chunks[4] = {8, 16, 32, 64};
     float best = 1e30f;
     int bt = h->threads, bl = h->layout, bc = h->chunk, bp = h->launch, br = h->rows;
