@@ -33,9 +33,9 @@
  * smallest needed (r1/2 z=96, 65,536 frames: 1.55 -> 1.32 ms; r5/6 z=96: 0.98
  * -> 0.89 ms). All arithmetic is fp32.
  *
- * Training (one frame per CTA of z threads): the forward pass runs all T
- * iterations, stores the posterior and the messages at every iteration
- * boundary (checkpoints) and the BCE loss mean over iterations, bits and
+ * Training (one frame at a time per CTA): the forward pass runs all T
+ * iterations and stores the posterior and the messages at the iteration
+ * boundaries (checkpoints); the loss is the BCE mean over iterations, bits and
  * frames (positive LLR = bit 1: loss = softplus(sg * P), sg = +1 for bit 0,
  * -1 for bit 1). The backward pass walks the iterations in reverse: it
  * restores iteration t's inputs from the checkpoints, recomputes its forward
@@ -43,8 +43,8 @@
  * Subgradients: sign() and the argmin choice are constant, d|x|/dx = sign(x),
  * relu'(0) = 0; edge e != i1 takes its magnitude from i1 (the first edge with
  * |L| == min1), edge i1 from i2 (the first other edge with |L| == min2).
- * Per-CTA weight gradients go to a per-frame partial array; a second kernel
- * reduces them in a fixed order (deterministic) and applies Adam.
+ * A CTA adds up the weight gradients of its frames; a second kernel adds the
+ * CTAs' in a fixed order (deterministic) and applies Adam.
  */
 #ifndef WLDPC_LMS_CUH
 #define WLDPC_LMS_CUH
@@ -301,10 +301,10 @@ lms_decode_kernel(const __grid_constant__ LmsArgs a)
 struct LmsTrainArgs {
     const float* llr;       /* frames x n */
     const uint8_t* cw;      /* frames x n transmitted bits (0/1) */
-    float* ck_post;         /* frames x T x n: posterior after iteration t */
-    float* ck_msg;          /* frames x (T-1) x E: messages after iteration t */
-    float* gpart;           /* frames x 2 x T x NBLK: per-frame weight gradient */
-    float* loss_part;       /* frames: per-frame loss */
+    float* ck_post;         /* per CTA T x n: posteriors after iteration t */
+    float* ck_msg;          /* per CTA T x E: messages after iteration t */
+    float* gpart;           /* per CTA 2 x T x NBLK: weight gradient over its frames */
+    double* loss_part;      /* per CTA: loss over its frames */
     const float* wa;        /* T x NBLK scales (device) */
     const float* wb;        /* T x NBLK offsets (device) */
     long long frames;
@@ -315,206 +315,268 @@ struct LmsTrainArgs {
 __device__ __forceinline__ float softplus_f(float x) { return x > 0.0f ? x + log1pf(__expf(-x)) : log1pf(__expf(x)); }
 __device__ __forceinline__ float sigmoid_f(float x) { return 1.0f / (1.0f + __expf(-x)); }
 
+/* One frame at a time per CTA of whole warps (lanes past z idle along). */
 template <int R, int Z>
 struct LmsTrainShape {
     static constexpr int MB = kMb[R];
     static constexpr int NBLK = num_blocks(R);
     static constexpr int N = kNB * Z;
     static constexpr int E = NBLK * Z;
-    /* P, M, L, gP, gM and the CTA's weight gradient */
-    static constexpr int SMEM = (2 * N + 3 * E + 2 * kLmsMaxIter * NBLK) * 4;
+    static constexpr int W = (Z + 31) / 32;
+    static constexpr int THREADS = 32 * W;
+    /* P, gP, gM, the CTA's weight gradient, the iteration's (a, b) pairs and
+     * its gradient per warp */
+    static constexpr int SMEM = (2 * N + E + 2 * kLmsMaxIter * NBLK + 2 * NBLK + W * 2 * NBLK) * 4;
+    /* 12 warps on an SM, as many as the shared memory allows at z = 96: up to
+     * 168 registers, one per message and the layer in work */
+    static constexpr int MIN_CTAS = 12 / W;
 };
 
-/* one layer of one iteration; optionally records L per edge */
-template <int R, int Z, int I, bool RECORD>
-__device__ __forceinline__ void lms_layer(float* P, float* M, float* Ls, const float* wa, const float* wb, int r)
+/* one iteration of the thread's rows on P; m: the messages, replaced by the
+ * new ones, or (RECORD) by the L they were turned into */
+template <int R, int Z, bool RECORD, int NBLK>
+__device__ __forceinline__ void lms_train_iteration(float* Pr, float* Prz, int r, bool owner, const float2* wab,
+                                                    float (&m)[NBLK])
 {
-    constexpr int d = layer_degree(R, I);
-    constexpr int b0 = block_index(R, I, 0);
-    float L[d];
-    uint32_t sgn = 0;
-    float m1 = __int_as_float(0x7f800000), m2 = __int_as_float(0x7f800000);
-    static_for<d>([&](auto E_) {
-        constexpr int e = decltype(E_)::value;
-        const float l = __fsub_rn(P[edge_var_c<R, Z, I, e>(r)], M[(b0 + e) * Z + r]);
-        L[e] = l;
-        if constexpr (RECORD) Ls[(b0 + e) * Z + r] = l;
-        sgn = __funnelshift_l(__float_as_uint(l), sgn, 1);
-        const float al = fabsf(l);
-        m2 = fminf(m2, fmaxf(m1, al));
-        m1 = fminf(m1, al);
-    });
-    const uint32_t fbo = ((uint32_t)((__popc(sgn) & 1) ^ (d & 1)) << 31) | 0x3f800000u;
-    static_for<d>([&](auto E_) {
-        constexpr int e = decltype(E_)::value;
-        const float l = L[e];
-        const float mu = (fabsf(l) == m1) ? m2 : m1;
-        const float mag = fmaxf(__fmaf_rn(wa[b0 + e], mu, -wb[b0 + e]), 0.0f);
-        const float msg = __fmul_rn(mag, __uint_as_float((__float_as_uint(l) & 0x80000000u) ^ fbo));
-        M[(b0 + e) * Z + r] = msg;
-        P[edge_var_c<R, Z, I, e>(r)] = __fadd_rn(l, msg);
+    static_for<kMb[R]>([&](auto I) {
+        constexpr int d = layer_degree(R, I);
+        constexpr int b0 = block_index(R, I, 0);
+        float L[d], A[d], mu[d];
+        uint32_t sgn = 0;
+        static_for<d>([&](auto E_) {
+            constexpr int e = decltype(E_)::value;
+            const float l = __fsub_rn(*edge_ptr<R, Z, I, e>(Pr, Prz, r), m[b0 + e]);
+            L[e] = l;
+            A[e] = fabsf(l);
+            sgn ^= __float_as_uint(l);
+        });
+        min_others<MinF32, d>(A, mu);
+        const uint32_t fbo = ((sgn ^ ((uint32_t)(d & 1) << 31)) & 0x80000000u) | 0x3f800000u;
+        static_for<d>([&](auto E_) {
+            constexpr int e = decltype(E_)::value;
+            const float l = L[e];
+            const float2 ab = wab[b0 + e];
+            const float mag = fmaxf(__fmaf_rn(ab.x, mu[e], -ab.y), 0.0f);
+            const float msg = __fmul_rn(mag, __uint_as_float((__float_as_uint(l) & 0x80000000u) ^ fbo));
+            m[b0 + e] = RECORD ? l : msg;
+            if (owner) *edge_ptr<R, Z, I, e>(Pr, Prz, r) = __fadd_rn(l, msg);
+        });
+        __syncthreads();
     });
 }
 
+/* K (a power of two, up to 32) sums over the warp at once: each step halves
+ * the values a lane holds and doubles the lanes they cover, K - 1 shuffles
+ * instead of 5 K. Lane l ends with value l / (32 / K). */
+template <int K>
+__device__ __forceinline__ float warp_sums(float (&v)[K], int lane)
+{
+    int bit = 16;
+#pragma unroll
+    for (int s = K / 2; s >= 1; s /= 2) {
+        const bool up = (lane & bit) != 0;
+#pragma unroll
+        for (int i = 0; i < s; i++) {
+            const float send = up ? v[i] : v[i + s], keep = up ? v[i + s] : v[i];
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, bit);
+        }
+        bit >>= 1;
+    }
+#pragma unroll
+    for (int o = 16 / K; o >= 1; o /= 2) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+    return v[0];
+}
+
+/* Loss and weight gradient. CTA c takes frames c, c + gridDim.x, ... What
+ * bounded the first form (one frame per launch of z threads, messages, their
+ * L and their gradient in shared memory: 6 warps on an SM; ten shuffles and
+ * two atomic additions per edge, per-thread atomics where z is no multiple of
+ * 32) was latency: 950 cycles per warp, edge and iteration. Here a thread's
+ * messages are registers, which the recomputed forward turns into the L that
+ * the backward pass reads, only the message gradients stay in shared memory,
+ * the rows' weight gradients are summed over a warp 16 or 32 at a time, and a
+ * CTA adds its frames' gradients up (fixed order) instead of writing each:
+ * a step of 4096 r1/2 z=96 frames 6.07 -> 1.81 ms.
+ * The last iteration is run once: its L are recorded on the way forward. */
 template <int R, int Z>
-__global__ void __launch_bounds__(Z)
+__global__ void __launch_bounds__(LmsTrainShape<R, Z>::THREADS, LmsTrainShape<R, Z>::MIN_CTAS)
 lms_train_kernel(const __grid_constant__ LmsTrainArgs a)
 {
     using S = LmsTrainShape<R, Z>;
-    constexpr int MB = S::MB, N = S::N, E = S::E, NBLK = S::NBLK;
+    constexpr int MB = S::MB, N = S::N, E = S::E, NBLK = S::NBLK, TH = S::THREADS, W = S::W;
     extern __shared__ __align__(128) float smem_tr[];
-    float* P = smem_tr;
-    float* gP = P + N;
-    float* M = gP + N;
-    float* Ls = M + E;
-    float* gM = Ls + E;
-    float* gW = gM + E;                          /* [2][T][NBLK] */
-    __shared__ float s_red[32];
+    float* const P = smem_tr;
+    float* const gP = P + N;
+    float* const gM = gP + N;
+    float* const gW = gM + E;                                       /* [2][T][NBLK] */
+    float2* const wab = reinterpret_cast<float2*>(gW + 2 * kLmsMaxIter * NBLK);
+    float* const part = reinterpret_cast<float*>(wab + NBLK);       /* [warp][2][NBLK] */
+    __shared__ double s_loss[W];
 
-    const int r = threadIdx.x;
-    const long long f = blockIdx.x;
-    if (f >= a.frames) return;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const bool owner = Z % 32 == 0 || tid < Z;
+    const int r = owner ? tid : tid % Z;
     const int T = a.iters;
-    const float* llr = a.llr + f * N;
-    const uint8_t* cw = a.cw + f * N;
-    float* ckp = a.ck_post + f * (long long)T * N;
-    float* ckm = a.ck_msg + f * (long long)(T > 1 ? T - 1 : 0) * E;
+    float* const Pr = P + r;
+    float* const Prz = Pr - Z;
+    float* const Gr = gP + r;
+    float* const Grz = Gr - Z;
+    float* const ckp = a.ck_post + blockIdx.x * (long long)T * N;
+    float* const ckm = a.ck_msg + blockIdx.x * (long long)T * E;
+    for (int q = tid; q < 2 * T * NBLK; q += TH) gW[q] = 0.0f;
+    double loss = 0.0;
 
-    for (int q = r; q < N; q += Z) { P[q] = llr[q]; gP[q] = 0.0f; }
-    for (int q = r; q < E; q += Z) { M[q] = 0.0f; gM[q] = 0.0f; }
-    for (int q = r; q < 2 * T * NBLK; q += Z) gW[q] = 0.0f;
-    __syncthreads();
-
-    /* forward: T iterations with checkpoints and the loss */
-    float loss = 0.0f;
-    for (int t = 0; t < T; t++) {
-        static_for<MB>([&](auto I) {
-            lms_layer<R, Z, decltype(I)::value, false>(P, M, nullptr, a.wa + t * NBLK, a.wb + t * NBLK, r);
-            __syncthreads();
-        });
-        for (int q = r; q < N; q += Z) {
-            const float p = P[q];
-            ckp[(long long)t * N + q] = p;
-            loss += softplus_f(cw[q] ? -p : p);
+    for (long long f = blockIdx.x; f < a.frames; f += gridDim.x) {
+        const float* const llr = a.llr + f * N;
+        const uint8_t* const cw = a.cw + f * N;
+        float m[NBLK];
+        __syncthreads();   /* the frame before is done with P, gP and gM */
+        for (int q = tid; q < N; q += TH) {
+            P[q] = llr[q];
+            gP[q] = 0.0f;
         }
-        if (t < T - 1)
-            for (int q = r; q < E; q += Z) ckm[(long long)t * E + q] = M[q];
-    }
-    /* block reduction of the loss (per thread into shared memory, then thread 0) */
-    for (int q = r; q < 32; q += Z) s_red[q] = 0.0f;
-    __syncthreads();
-    atomicAdd(&s_red[r & 31], loss);
-    __syncthreads();
-    if (r == 0) {
-        float s = 0.0f;
-        for (int q = 0; q < 32; q++) s += s_red[q];
-        a.loss_part[f] = s * a.inv_norm;
-    }
-    __syncthreads();
+        for (int q = tid; q < E; q += TH) gM[q] = 0.0f;
+#pragma unroll
+        for (int q = 0; q < NBLK; q++) m[q] = 0.0f;
+        auto weights = [&](int t) {   /* between two barriers */
+            for (int q = tid; q < NBLK; q += TH) wab[q] = make_float2(a.wa[t * NBLK + q], a.wb[t * NBLK + q]);
+        };
 
-    /* backward */
-    for (int t = T - 1; t >= 0; t--) {
-        /* restore the inputs of iteration t and recompute it, keeping L */
-        const float* pin = t == 0 ? llr : ckp + (long long)(t - 1) * N;
-        for (int q = r; q < N; q += Z) P[q] = pin[q];
-        for (int q = r; q < E; q += Z) M[q] = t == 0 ? 0.0f : ckm[(long long)(t - 1) * E + q];
-        __syncthreads();
-        static_for<MB>([&](auto I) {
-            lms_layer<R, Z, decltype(I)::value, true>(P, M, Ls, a.wa + t * NBLK, a.wb + t * NBLK, r);
+        /* forward, keeping what each iteration ends with except the last two:
+         * the last but one leads straight into the last */
+        for (int t = 0; t < T - 1; t++) {
+            weights(t);
             __syncthreads();
-        });
-        /* loss gradient at the end of iteration t */
-        for (int q = r; q < N; q += Z) {
-            const float p = P[q];
-            const float sg = cw[q] ? -1.0f : 1.0f;
-            gP[q] += sg * sigmoid_f(sg * p) * a.inv_norm;
+            lms_train_iteration<R, Z, false>(Pr, Prz, r, owner, wab, m);
+            if (t < T - 2) {
+                for (int q = tid; q < N; q += TH) ckp[(long long)t * N + q] = P[q];
+                if (owner) {
+#pragma unroll
+                    for (int q = 0; q < NBLK; q++) ckm[(long long)t * E + q * Z + r] = m[q];
+                }
+            }
         }
-        __syncthreads();
-        static_for<MB>([&](auto IR) {
-            constexpr int I = MB - 1 - decltype(IR)::value;
-            constexpr int d = layer_degree(R, I);
-            constexpr int b0 = block_index(R, I, 0);
-            float L[d], gL[d];
-            float m1 = __int_as_float(0x7f800000), m2 = __int_as_float(0x7f800000);
-            uint32_t negpar = (uint32_t)(d & 1);   /* odd-degree rows flip the extrinsic sign */
-            static_for<d>([&](auto E_) {
-                constexpr int e = decltype(E_)::value;
-                L[e] = Ls[(b0 + e) * Z + r];
-                gL[e] = gP[edge_var_c<R, Z, I, e>(r)];
-                negpar ^= __float_as_uint(L[e]) >> 31;
-                const float al = fabsf(L[e]);
-                m2 = fminf(m2, fmaxf(m1, al));
-                m1 = fminf(m1, al);
-            });
-            int i1 = -1, i2 = -1;
-            static_for<d>([&](auto E_) {
-                constexpr int e = decltype(E_)::value;
-                if (i1 < 0 && fabsf(L[e]) == m1) i1 = e;
-            });
-            static_for<d>([&](auto E_) {
-                constexpr int e = decltype(E_)::value;
-                if (i2 < 0 && e != i1 && fabsf(L[e]) == m2) i2 = e;
-            });
-            float g_to_i1 = 0.0f, g_to_i2 = 0.0f;
-            static_for<d>([&](auto E_) {
-                constexpr int e = decltype(E_)::value;
-                const float l = L[e];
-                const bool is_i1 = (e == i1);
-                const float mu = (fabsf(l) == m1) ? m2 : m1;
-                const float wa = a.wa[t * NBLK + b0 + e], wb = a.wb[t * NBLK + b0 + e];
-                const float pre = __fmaf_rn(wa, mu, -wb);
-                const float s = ((negpar ^ (__float_as_uint(l) >> 31)) & 1u) ? -1.0f : 1.0f;
-                const float G = gL[e] + gM[(b0 + e) * Z + r];
-                float ga = 0.0f, gb = 0.0f;
-                if (pre > 0.0f) {
-                    ga = G * s * mu;
-                    gb = -G * s;
-                    const float gmu = G * s * wa;
-                    if (is_i1) g_to_i2 += gmu;
+
+        /* backward; P and m hold iteration t's inputs, from the checkpoint
+         * after iteration t - 1 except for the last */
+        float floss = 0.0f;
+        for (int t = T - 1; t >= 0; t--) {
+            if (t < T - 1) {
+                const float* const pin = t == 0 ? llr : ckp + (long long)(t - 1) * N;
+                for (int q = tid; q < N; q += TH) P[q] = pin[q];
+#pragma unroll
+                for (int q = 0; q < NBLK; q++) m[q] = t == 0 ? 0.0f : ckm[(long long)(t - 1) * E + q * Z + r];
+            }
+            weights(t);
+            __syncthreads();
+            lms_train_iteration<R, Z, true>(Pr, Prz, r, owner, wab, m);   /* m: L from here */
+            /* loss of iteration t and its gradient */
+            for (int q = tid; q < N; q += TH) {
+                const float p = P[q];
+                const float sg = cw[q] ? -1.0f : 1.0f;
+                floss += softplus_f(sg * p);
+                gP[q] += sg * sigmoid_f(sg * p) * a.inv_norm;
+            }
+            __syncthreads();
+            static_for<MB>([&](auto IR) {
+                constexpr int I = MB - 1 - decltype(IR)::value;
+                constexpr int d = layer_degree(R, I);
+                constexpr int b0 = block_index(R, I, 0);
+                float L[d], gL[d];
+                uint32_t negpar = (uint32_t)(d & 1) << 31;   /* odd-degree rows flip the extrinsic sign */
+                static_for<d>([&](auto E_) {
+                    constexpr int e = decltype(E_)::value;
+                    L[e] = m[b0 + e];
+                    gL[e] = *edge_ptr<R, Z, I, e>(Gr, Grz, r);
+                    negpar ^= __float_as_uint(L[e]);
+                });
+                float m1, m2;
+                two_min_abs<0, d>(L, m1, m2);
+                /* i1: the first edge with |L| == m1, i2: the first other one with |L| == m2 */
+                int i1 = 0, i2 = 0;
+                static_for<d>([&](auto E_) {
+                    constexpr int e = d - 1 - decltype(E_)::value;
+                    i1 = fabsf(L[e]) == m1 ? e : i1;
+                });
+                static_for<d>([&](auto E_) {
+                    constexpr int e = d - 1 - decltype(E_)::value;
+                    i2 = fabsf(L[e]) == m2 && e != i1 ? e : i2;
+                });
+                constexpr int K = 2 * d <= 16 ? 16 : 32;
+                constexpr int H = (2 * d + K - 1) / K;    /* groups of K sums (2 for d = 20) */
+                float v[H][K];
+#pragma unroll
+                for (int h = 0; h < H; h++)
+#pragma unroll
+                    for (int q = 0; q < K; q++) v[h][q] = 0.0f;
+                float g_to_i1 = 0.0f, g_to_i2 = 0.0f;
+                static_for<d>([&](auto E_) {
+                    constexpr int e = decltype(E_)::value;
+                    const float mu = (fabsf(L[e]) == m1) ? m2 : m1;
+                    const float2 ab = wab[b0 + e];
+                    const float pre = __fmaf_rn(ab.x, mu, -ab.y);
+                    const float G = owner ? gL[e] + gM[(b0 + e) * Z + r] : 0.0f;
+                    /* gradient of the magnitude, zero where relu cut it off */
+                    const float gs = pre > 0.0f ? __uint_as_float(__float_as_uint(G) ^ ((negpar ^ __float_as_uint(L[e])) &
+                                                                                       0x80000000u))
+                                                : 0.0f;
+                    v[e / K][e % K] = gs * mu;
+                    v[(d + e) / K][(d + e) % K] = -gs;
+                    const float gmu = gs * ab.x;
+                    if (e == i1) g_to_i2 += gmu;
                     else g_to_i1 += gmu;
-                }
-                /* reduce over the rows of this block (the CTA's z threads):
-                 * whole warps shuffle, a partial last warp adds per thread */
-                if constexpr (Z % 32 == 0) {
-                    for (int o = 16; o > 0; o >>= 1) {
-                        ga += __shfl_xor_sync(0xffffffffu, ga, o);
-                        gb += __shfl_xor_sync(0xffffffffu, gb, o);
+                });
+                static_for<d>([&](auto E_) {
+                    constexpr int e = decltype(E_)::value;
+                    const float sgn_l = __uint_as_float((__float_as_uint(L[e]) & 0x80000000u) | 0x3f800000u);
+                    float g = gL[e];
+                    if (e == i1) g += g_to_i1 * sgn_l;
+                    if (e == i2) g += g_to_i2 * sgn_l;
+                    if (owner) {
+                        *edge_ptr<R, Z, I, e>(Gr, Grz, r) = g;
+                        gM[(b0 + e) * Z + r] = -g;
                     }
-                    if ((r & 31) == 0) {
-                        atomicAdd(&gW[t * NBLK + b0 + e], ga);
-                        atomicAdd(&gW[(T + t) * NBLK + b0 + e], gb);
-                    }
-                } else if (ga != 0.0f || gb != 0.0f) {
-                    atomicAdd(&gW[t * NBLK + b0 + e], ga);
-                    atomicAdd(&gW[(T + t) * NBLK + b0 + e], gb);
+                });
+#pragma unroll
+                for (int h = 0; h < H; h++) {
+                    const float sum = warp_sums<K>(v[h], lane);
+                    const int k = h * K + lane / (32 / K);
+                    if (lane % (32 / K) == 0 && k < 2 * d)
+                        part[warp * 2 * NBLK + (k < d ? b0 + k : NBLK + b0 + k - d)] = sum;
                 }
+                __syncthreads();
             });
-            static_for<d>([&](auto E_) {
-                constexpr int e = decltype(E_)::value;
-                const float sgn_l = (__float_as_uint(L[e]) >> 31) ? -1.0f : 1.0f;
-                float g = gL[e];
-                if (e == i1) g += g_to_i1 * sgn_l;
-                if (e == i2) g += g_to_i2 * sgn_l;
-                gP[edge_var_c<R, Z, I, e>(r)] = g;
-                gM[(b0 + e) * Z + r] = -g;
-            });
-            __syncthreads();
-        });
+            for (int q = tid; q < 2 * NBLK; q += TH) {
+                float g = part[q];
+                for (int w = 1; w < W; w++) g += part[w * 2 * NBLK + q];
+                gW[q < NBLK ? t * NBLK + q : (T + t) * NBLK + q - NBLK] += g;
+            }
+        }
+        loss += (double)floss;
     }
-    for (int q = r; q < 2 * T * NBLK; q += Z) a.gpart[f * 2 * T * NBLK + q] = gW[q];
+    /* the CTA's loss and gradient */
+    for (int o = 16; o > 0; o >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, o);
+    if (lane == 0) s_loss[warp] = loss;
+    __syncthreads();
+    if (tid == 0) {
+        double sum = 0.0;
+        for (int w = 0; w < W; w++) sum += s_loss[w];
+        a.loss_part[blockIdx.x] = sum * (double)a.inv_norm;
+    }
+    for (int q = tid; q < 2 * T * NBLK; q += TH) a.gpart[(long long)blockIdx.x * 2 * T * NBLK + q] = gW[q];
 }
 
-/* Column sums of the per-frame gradients in frame order, then Adam. One
- * thread per weight; w holds a then b, [T][NBLK] each. */
+/* Column sums of the CTAs' gradients in a fixed order, then Adam; w holds a
+ * then b, [T][NBLK] each. */
 struct AdamArgs {
-    const float* gpart;      /* frames x nw */
-    const float* loss_part;  /* frames */
+    const float* gpart;      /* rows x nw */
+    const double* loss_part; /* rows */
     float* grad;             /* nw, written (the reduced gradient) */
     float* w;                /* nw parameters */
     float* m;                /* nw first moments */
     float* v;                /* nw second moments */
     float* loss_out;         /* one float: the batch loss, or null */
-    long long frames;
+    int rows;                /* CTAs of the training launch, or 1 */
     int nw;
     int step;                /* 1-based Adam step */
     float lr, beta1, beta2, eps;

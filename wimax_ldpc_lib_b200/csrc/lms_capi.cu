@@ -34,19 +34,39 @@ WLDPC_LMS_HALVES(4)
 WLDPC_LMS_HALVES(5)
 #undef WLDPC_LMS_HALVES
 
-/* Column sums of the per-frame gradients in frame order (deterministic),
- * the batch loss, then Adam; one thread per weight. */
-__global__ void lms_reduce_adam_kernel(const __grid_constant__ AdamArgs a)
+/* Column sums of the CTAs' gradients (deterministic), the batch loss, then
+ * Adam. A block takes 32 weights; its 16 warps add every 16th row (one thread
+ * per weight walking all rows, one after the other, waited for each), then
+ * the 16 sums in order. */
+constexpr int kReduceRows = 16;
+__global__ void __launch_bounds__(32 * kReduceRows) lms_reduce_adam_kernel(const __grid_constant__ AdamArgs a)
 {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j == 0 && a.loss_out) {
-        float s = 0.0f;
-        for (long long f = 0; f < a.frames; f++) s += a.loss_part[f];
-        *a.loss_out = s;
-    }
-    if (j >= a.nw) return;
+    __shared__ float s_sum[kReduceRows][32];
+    __shared__ double s_loss[kReduceRows];
+    const int lane = threadIdx.x & 31, row0 = threadIdx.x >> 5;
+    const int j = blockIdx.x * 32 + lane;
     float g = 0.0f;
-    for (long long f = 0; f < a.frames; f++) g += a.gpart[f * a.nw + j];
+    if (j < a.nw) {
+#pragma unroll 4
+        for (int q = row0; q < a.rows; q += kReduceRows) g += a.gpart[(long long)q * a.nw + j];
+    }
+    s_sum[row0][lane] = g;
+    const bool with_loss = blockIdx.x == 0 && a.loss_out;
+    if (with_loss) {
+        double s = 0.0;
+        for (int q = (int)threadIdx.x; q < a.rows; q += 32 * kReduceRows) s += a.loss_part[q];
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        if (lane == 0) s_loss[row0] = s;
+    }
+    __syncthreads();
+    if (with_loss && threadIdx.x == 32) {
+        double s = 0.0;
+        for (int q = 0; q < kReduceRows; q++) s += s_loss[q];
+        *a.loss_out = (float)s;
+    }
+    if (row0 != 0 || j >= a.nw) return;
+    g = s_sum[0][lane];
+    for (int q = 1; q < kReduceRows; q++) g += s_sum[q][lane];
     a.grad[j] = g;
     if (!a.apply) return;
     const float m = a.beta1 * a.m[j] + (1.0f - a.beta1) * g;
@@ -122,6 +142,7 @@ struct wldpc_lms {
     cudaStream_t pipe[kHostStages] = {};
     cudaEvent_t ev_user = nullptr;                     /* orders the handle's stream after a caller's */
     int adam_step = 0;
+    int train_ctas = 0;                                /* CTAs of a training launch that fit the GPU at once */
 };
 
 static int lms_sync_host_weights(wldpc_lms* h)
@@ -426,14 +447,26 @@ int wldpc_lms_decode_host_hard(wldpc_lms* h, const float* llr, int8_t* decoded, 
 }
 
 /* one training forward/backward over `frames` frames already on the device;
- * leaves the per-frame partials in h->gpart / h->lpart */
-static int lms_forward_backward(wldpc_lms* h, const float* llr, const uint8_t* cw, size_t frames, cudaStream_t st)
+ * leaves *rows partial gradients and losses in h->gpart / h->lpart */
+static int lms_forward_backward(wldpc_lms* h, const float* llr, const uint8_t* cw, size_t frames, cudaStream_t st,
+                                int* rows)
 {
     const size_t n = (size_t)h->code.n, E = (size_t)h->nblk * h->z, T = (size_t)h->T;
     const size_t nw = 2 * T * h->nblk;
+    const LmsLaunch* k = h->k;
     int rc;
-    if ((rc = h->ckp.reserve(frames * T * n * 4)) || (rc = h->ckm.reserve(frames * (T > 1 ? T - 1 : 1) * E * 4)) ||
-        (rc = h->gpart.reserve(frames * nw * 4)) || (rc = h->lpart.reserve(frames * 4)))
+    if (h->train_ctas == 0) {
+        int dev = 0, sms = 0, per = 0;
+        CU(cudaFuncSetAttribute(k->train, cudaFuncAttributeMaxDynamicSharedMemorySize, k->train_smem));
+        CU(cudaGetDevice(&dev));
+        CU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+        CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k->train, k->train_threads, k->train_smem));
+        h->train_ctas = sms * (per > 0 ? per : 1);
+    }
+    const size_t ctas = frames < (size_t)h->train_ctas ? frames : (size_t)h->train_ctas;
+    *rows = (int)ctas;
+    if ((rc = h->ckp.reserve(ctas * T * n * 4)) || (rc = h->ckm.reserve(ctas * T * E * 4)) ||
+        (rc = h->gpart.reserve(ctas * nw * 4)) || (rc = h->lpart.reserve(ctas * 8)))
         return rc;
     LmsTrainArgs a;
     a.llr = llr;
@@ -441,31 +474,28 @@ static int lms_forward_backward(wldpc_lms* h, const float* llr, const uint8_t* c
     a.ck_post = (float*)h->ckp.p;
     a.ck_msg = (float*)h->ckm.p;
     a.gpart = (float*)h->gpart.p;
-    a.loss_part = (float*)h->lpart.p;
+    a.loss_part = (double*)h->lpart.p;
     a.wa = (const float*)h->wdev.p;
     a.wb = (const float*)h->wdev.p + T * h->nblk;
     a.frames = (long long)frames;
     a.iters = h->T;
     a.inv_norm = (float)(1.0 / ((double)T * (double)n * (double)frames));
-    const LmsLaunch* k = h->k;
-    if (k->train_smem > 48 * 1024)
-        CU(cudaFuncSetAttribute(k->train, cudaFuncAttributeMaxDynamicSharedMemorySize, k->train_smem));
-    k->train<<<(unsigned)frames, h->z, k->train_smem, st>>>(a);
+    k->train<<<(unsigned)ctas, k->train_threads, k->train_smem, st>>>(a);
     CU(cudaGetLastError());
     return WLDPC_OK;
 }
 
-static int lms_reduce(wldpc_lms* h, size_t frames, int apply, float lr, float* loss_out, cudaStream_t st)
+static int lms_reduce(wldpc_lms* h, int rows, int apply, float lr, float* loss_out, cudaStream_t st)
 {
     AdamArgs a;
     a.gpart = (const float*)h->gpart.p;
-    a.loss_part = (const float*)h->lpart.p;
+    a.loss_part = (const double*)h->lpart.p;
     a.grad = (float*)h->grad.p;
     a.w = (float*)h->wdev.p;
     a.m = (float*)h->mdev.p;
     a.v = (float*)h->vdev.p;
     a.loss_out = loss_out;
-    a.frames = (long long)frames;
+    a.rows = rows;
     a.nw = 2 * h->T * h->nblk;
     a.step = h->adam_step + 1;
     a.lr = lr;
@@ -473,7 +503,7 @@ static int lms_reduce(wldpc_lms* h, size_t frames, int apply, float lr, float* l
     a.beta2 = 0.999f;
     a.eps = 1e-8f;
     a.apply = apply;
-    lms_reduce_adam_kernel<<<(a.nw + 127) / 128, 128, 0, st>>>(a);
+    lms_reduce_adam_kernel<<<(a.nw + 31) / 32, 32 * kReduceRows, 0, st>>>(a);
     CU(cudaGetLastError());
     if (apply) {
         h->adam_step++;
@@ -491,14 +521,14 @@ int wldpc_lms_loss_grad(wldpc_lms* h, const float* llr, const uint8_t* codeword,
         if (rc) return rc;
     }
     const size_t n = (size_t)h->code.n;
-    int rc;
+    int rc, rows = 0;
     if ((rc = h->tllr.reserve(frames * n * 4)) || (rc = h->tcw.reserve(frames * n)) || (rc = h->loss.reserve(4)))
         return rc;
     CU(cudaMemcpyAsync(h->tllr.p, llr, frames * n * 4, cudaMemcpyHostToDevice, h->stream));
     CU(cudaMemcpyAsync(h->tcw.p, codeword, frames * n, cudaMemcpyHostToDevice, h->stream));
-    if ((rc = lms_forward_backward(h, (const float*)h->tllr.p, (const uint8_t*)h->tcw.p, frames, h->stream)))
+    if ((rc = lms_forward_backward(h, (const float*)h->tllr.p, (const uint8_t*)h->tcw.p, frames, h->stream, &rows)))
         return rc;
-    if ((rc = lms_reduce(h, frames, 0, 0.0f, (float*)h->loss.p, h->stream))) return rc;
+    if ((rc = lms_reduce(h, rows, 0, 0.0f, (float*)h->loss.p, h->stream))) return rc;
     const size_t nw = (size_t)2 * h->T * h->nblk;
     std::vector<float> g(nw);
     float l = 0.0f;
@@ -527,7 +557,7 @@ int wldpc_lms_train(wldpc_lms* h, unsigned steps, unsigned batch, float ebno_lo_
         if (rc) return rc;
     }
     const size_t n = (size_t)h->code.n;
-    int rc;
+    int rc, rows = 0;
     if ((rc = h->tllr.reserve((size_t)batch * n * 4)) || (rc = h->tcw.reserve((size_t)batch * n)) ||
         (rc = h->loss.reserve((size_t)(steps ? steps : 1) * 4)))
         return rc;
@@ -545,9 +575,9 @@ int wldpc_lms_train(wldpc_lms* h, unsigned steps, unsigned batch, float ebno_lo_
         } else {
             CU(launch_framegen(h->code, f, h->stream));
         }
-        if ((rc = lms_forward_backward(h, (const float*)h->tllr.p, (const uint8_t*)h->tcw.p, batch, h->stream)))
+        if ((rc = lms_forward_backward(h, (const float*)h->tllr.p, (const uint8_t*)h->tcw.p, batch, h->stream, &rows)))
             return rc;
-        if ((rc = lms_reduce(h, batch, 1, lr, (float*)h->loss.p + s, h->stream))) return rc;
+        if ((rc = lms_reduce(h, rows, 1, lr, (float*)h->loss.p + s, h->stream))) return rc;
     }
     if (loss_history && steps) CU(cudaMemcpyAsync(loss_history, h->loss.p, (size_t)steps * 4, cudaMemcpyDeviceToHost, h->stream));
     CU(cudaStreamSynchronize(h->stream));
@@ -579,7 +609,7 @@ int wldpc_lms_step_grad(wldpc_lms* h, unsigned batch, float ebno_lo_db, float eb
         if (rc) return rc;
     }
     const size_t n = (size_t)h->code.n, nw = (size_t)2 * h->T * h->nblk;
-    int rc;
+    int rc, rows = 0;
     if ((rc = h->tllr.reserve((size_t)batch * n * 4)) || (rc = h->tcw.reserve((size_t)batch * n)) ||
         (rc = h->loss.reserve(4)))
         return rc;
@@ -597,9 +627,9 @@ int wldpc_lms_step_grad(wldpc_lms* h, unsigned batch, float ebno_lo_db, float eb
     } else {
         CU(launch_framegen(h->code, f, h->stream));
     }
-    if ((rc = lms_forward_backward(h, (const float*)h->tllr.p, (const uint8_t*)h->tcw.p, batch, h->stream)))
+    if ((rc = lms_forward_backward(h, (const float*)h->tllr.p, (const uint8_t*)h->tcw.p, batch, h->stream, &rows)))
         return rc;
-    if ((rc = lms_reduce(h, batch, 0, 0.0f, (float*)h->loss.p, h->stream))) return rc;
+    if ((rc = lms_reduce(h, rows, 0, 0.0f, (float*)h->loss.p, h->stream))) return rc;
     CU(cudaMemcpyAsync(grad, h->grad.p, nw * 4, cudaMemcpyDeviceToDevice, h->stream));
     if (loss) CU(cudaMemcpyAsync(loss, h->loss.p, 4, cudaMemcpyDeviceToDevice, h->stream));
     CU(cudaStreamSynchronize(h->stream));
@@ -616,14 +646,14 @@ int wldpc_lms_apply_grad(wldpc_lms* h, const float* grad, float lr, void* stream
     int rc;
     if ((rc = lms_after_user_stream(h, (cudaStream_t)stream))) return rc;
     AdamArgs a;
-    a.gpart = grad;            /* one "frame": the given gradient */
+    a.gpart = grad;            /* one row: the given gradient */
     a.loss_part = nullptr;
     a.grad = (float*)h->grad.p;
     a.w = (float*)h->wdev.p;
     a.m = (float*)h->mdev.p;
     a.v = (float*)h->vdev.p;
     a.loss_out = nullptr;
-    a.frames = 1;
+    a.rows = 1;
     a.nw = 2 * h->T * h->nblk;
     a.step = h->adam_step + 1;
     a.lr = lr;
@@ -631,7 +661,7 @@ int wldpc_lms_apply_grad(wldpc_lms* h, const float* grad, float lr, void* stream
     a.beta2 = 0.999f;
     a.eps = 1e-8f;
     a.apply = 1;
-    lms_reduce_adam_kernel<<<(a.nw + 127) / 128, 128, 0, h->stream>>>(a);
+    lms_reduce_adam_kernel<<<(a.nw + 31) / 32, 32 * kReduceRows, 0, h->stream>>>(a);
     CU(cudaGetLastError());
     h->adam_step++;
     h->host_stale = true;

@@ -17,7 +17,7 @@ struct LmsLaunch {
     void (*decode)(const LmsArgs);
     int threads, frames_per_cta, smem;
     void (*train)(const LmsTrainArgs);
-    int train_smem;          /* train CTA = z threads, one frame */
+    int train_smem, train_threads;
     void (*decode16)(const Lms16Args);   /* packed-half decoder (lms16.cuh) */
     int threads16, frames16;             /* its CTA size and frames per CTA (static shared memory) */
     UnitLaunch<LmsArgs> unit;            /* large batches */

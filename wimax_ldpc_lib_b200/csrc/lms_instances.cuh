@@ -17,7 +17,8 @@ namespace wldpc {
 #define WLDPC_LMS_ENTRY(Z)                                                                                     \
     {Z, &lms_decode_kernel<WLDPC_LMS_RATE, Z>, LmsShape<WLDPC_LMS_RATE, Z>::THREADS,                           \
      LmsShape<WLDPC_LMS_RATE, Z>::G, LmsShape<WLDPC_LMS_RATE, Z>::SMEM, &lms_train_kernel<WLDPC_LMS_RATE, Z>, \
-     LmsTrainShape<WLDPC_LMS_RATE, Z>::SMEM, &lms16_decode_kernel<WLDPC_LMS_RATE, Z>,                         \
+     LmsTrainShape<WLDPC_LMS_RATE, Z>::SMEM, LmsTrainShape<WLDPC_LMS_RATE, Z>::THREADS,                       \
+     &lms16_decode_kernel<WLDPC_LMS_RATE, Z>,                                                                 \
      Lms16Shape<WLDPC_LMS_RATE, Z>::THREADS, Lms16Shape<WLDPC_LMS_RATE, Z>::FRAMES,                          \
      unit_launch<WLDPC_LMS_RATE, Z, LearnedRow>(), unit_launch16<WLDPC_LMS_RATE, Z>()}
 
