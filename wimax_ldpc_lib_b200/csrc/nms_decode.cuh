@@ -59,6 +59,7 @@ struct DecodeArgs {
     long long frames;
     int max_iter;
     unsigned wait_limit_us = kWaitLimitUs;   /* bound of the staging wait (the drain wait after a timeout is full) */
+    bool direct = false;    /* llr is pinned host memory: staged by ordinary loads, nothing to wait for */
     /* used only by the kernels whose z is a run-time value (ZT == 0): */
     int z;
     unsigned short shift[96];   /* per non-zero block, row-major over base rows */
@@ -343,16 +344,35 @@ tdmp_decode_kernel(const __grid_constant__ DecodeArgs a)
         s_last[1] = 0;
         s_half[0] = 0;
         s_half[1] = 0;
-        const uint32_t bytes = (uint32_t)(nf * N * 4);
-        mbar_arrive_expect_tx(&bar, bytes);
-        bulk_g2s(smem_post, a.llr + f0 * N, bytes, &bar);
+        if (!a.direct) {
+            const uint32_t bytes = (uint32_t)(nf * N * 4);
+            mbar_arrive_expect_tx(&bar, bytes);
+            bulk_g2s(smem_post, a.llr + f0 * N, bytes, &bar);
+        }
     }
-    __syncthreads();
-    const bool ok = mbar_wait_bounded(&bar, 0, a.wait_limit_us);
+    bool ok = a.wait_limit_us != 0;
+    if (a.direct) {
+        /* every load in flight at once: one trip over the bus */
+        const float4* const src = reinterpret_cast<const float4*>(a.llr + f0 * N);
+        float4 x[6];
+#pragma unroll
+        for (int s = 0; s < 6; s++) {
+            const int v = tid + s * nthreads;
+            if (v < nf * N / 4) x[s] = __ldcv(src + v);
+        }
+#pragma unroll
+        for (int s = 0; s < 6; s++) {
+            const int v = tid + s * nthreads;
+            if (v < nf * N / 4) reinterpret_cast<float4*>(smem_post)[v] = x[s];
+        }
+    } else {
+        __syncthreads();
+        ok = mbar_wait_bounded(&bar, 0, a.wait_limit_us);
+    }
     if (__syncthreads_or(!ok)) {
         if (tid == 0) {
             atomicOr(a.err, kErrWaitTimeout);
-            mbar_wait_bounded(&bar, 0, kWaitLimitUs);   /* let an in-flight copy land before exit */
+            if (!a.direct) mbar_wait_bounded(&bar, 0, kWaitLimitUs);   /* let an in-flight copy land before exit */
         }
         return;
     }

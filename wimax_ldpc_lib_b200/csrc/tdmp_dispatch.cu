@@ -27,7 +27,7 @@ cudaError_t launch_tdmp(int rate, int z, int mode, const DecodeArgs& args, cudaS
     const TdmpLaunch* e = tdmp_entry(rate, z, mode);
     if (!e) return cudaErrorInvalidValue;
     if (args.frames <= 0) return cudaSuccess;
-    if (unit_takes(e->unit, args.frames)) return launch_unit(e->unit, args, st);
+    if (!args.direct && unit_takes(e->unit, args.frames)) return launch_unit(e->unit, args, st);
     DecodeArgs a = args;
     int threads = e->threads, smem = e->smem;
     if (e->runtime_z) {
