@@ -378,15 +378,23 @@ const EncLanesLaunch* enc_lanes_entry(int rate, int z)
     return &tables[rate][z_index(z)];
 }
 
+/* Frames per warp of the lane-per-frame encoder: 4, whose loads are all issued
+ * at once, or 8, which spread phase B's fixed work over more of them, where
+ * frames are short and the batch fills the GPU with 8 (148 SMs x 4 warps).
+ * Timed at 2 to 32 per warp, seven codes, 600 to 262,144 frames (us, 4 / 8):
+ * z=96 141 / 148, z=64 96 / 100, z=60 113 / 119, z=48 82 / 76, z=24 52 / 45 at
+ * 262,144; z=24 7 / 9 at 4096. */
+static int encode_per_warp(int z, long long frames) { return z >= 60 || frames <= 148 * 4 * 8 ? 4 : 8; }
+
 cudaError_t launch_encode_bytes(const CodeDesc& c, const uint8_t* info, uint8_t* cw, long long frames,
                                 cudaStream_t st)
 {
     if (frames <= 0) return cudaSuccess;
     const EncLanesLaunch* e = enc_lanes_entry(c.rate, c.z);
     if (e && ((uintptr_t)info % e->align) == 0 && ((uintptr_t)cw % e->align) == 0) {
-        const long long frames_per_cta = e->threads;   /* one frame per thread */
-        e->kernel<<<(unsigned)((frames + frames_per_cta - 1) / frames_per_cta), e->threads, 0, st>>>(info, cw,
-                                                                                                   frames);
+        const int per_warp = encode_per_warp(c.z, frames);
+        const long long per_cta = (long long)(e->threads / 32) * per_warp;
+        e->kernel<<<(unsigned)((frames + per_cta - 1) / per_cta), e->threads, 0, st>>>(info, cw, frames, per_warp);
         return cudaGetLastError();
     }
     const long long blocks = (frames + kEncWarps - 1) / kEncWarps;

@@ -39,9 +39,9 @@ cudaError_t launch_framegen_nullspace(const CodeDesc& c, const FramegenArgs& a, 
 /* encoder specialised on (rate, z), one frame per lane (encode_lanes.cuh);
  * info and codeword must be aligned to `align` bytes */
 struct EncLanesLaunch {
-    void (*kernel)(const uint8_t*, uint8_t*, long long);
+    void (*kernel)(const uint8_t*, uint8_t*, long long, int);
     int align;
-    int threads;        /* per CTA: 32 frames per warp */
+    int threads;        /* per CTA */
 };
 /* entry for (rate, z) or null (rate 3/4B has no encoder) */
 const EncLanesLaunch* enc_lanes_entry(int rate, int z);

@@ -4,7 +4,8 @@
  * reference ldpc_encoder::encode_data (reference lib/ldpc_encoder.cc:29-105);
  * the block recursion is the one written out in encode.cuh.
  *
- * A warp encodes 32 frames in three phases:
+ * A warp encodes 4 or 8 frames (the launch says which, encode_per_warp()) in
+ * three phases:
  *  A. per frame, the whole warp reads the k info bytes in 16-byte (or 8-byte)
  *     chunks, coalesced, copies them to the systematic part of the codeword
  *     (reference :90, so non-0/1 bytes pass through) and packs them into bits
@@ -17,8 +18,17 @@
  *     one contiguous bit array to the frame's output row;
  *  C. per frame, the whole warp expands the parity bits to bytes and stores
  *     them in 16-byte (or 8-byte) chunks, coalesced.
- * Rows are an odd number of words apart, so lane-per-frame accesses hit 32
+ * Rows are an odd number of words apart, so lane-per-frame accesses hit
  * different banks.
+ *
+ * What binds is HBM. With 32 frames per warp the lanes of phase B were all
+ * busy, but the rows took 29 KB of shared memory per CTA, out of the L1 whose
+ * lines the loads in flight need: 262,144 r1/2 z=96 frames 191 us. With rows
+ * for 8 frames 151 us at the same 24 warps per SM, with the systematic bytes
+ * stored streaming like the parity 141 us, 0.98 of the measured copy
+ * bandwidth; phase B's idle lanes cost issue slots that were free (34% used).
+ * r1/2 z=24: 52 -> 45 us. A batch of 4096 frames now spreads over all SMs:
+ * 15.8 -> 9.4 us.
  */
 #ifndef WLDPC_ENCODE_LANES_CUH
 #define WLDPC_ENCODE_LANES_CUH
@@ -44,7 +54,8 @@ struct EncLanes {
     static constexpr int CB = (K % 16 == 0) ? 16 : 8;   /* bytes per lane per memory chunk */
     static constexpr int WARPS = 4;
     static constexpr int THREADS = 32 * WARPS;
-    static constexpr int SMEM_WORDS = WARPS * 32 * (UROW + OROW);
+    static constexpr int ROWS = 8;                      /* frames per warp, at most */
+    static constexpr int SMEM_WORDS = WARPS * ROWS * (UROW + OROW);
     static constexpr int D = D_of(R, Z), X = kX[R];
 };
 
@@ -90,18 +101,19 @@ __device__ __forceinline__ uint32_t rot32_at(Get&& get)
 
 template <int R, int Z>
 __global__ void __launch_bounds__(EncLanes<R, Z>::THREADS)
-encode_lanes_kernel(const uint8_t* __restrict__ info, uint8_t* __restrict__ cw, long long frames)
+encode_lanes_kernel(const uint8_t* __restrict__ info, uint8_t* __restrict__ cw, long long frames,
+                    int per_warp /* 1 .. ROWS */)
 {
     using S = EncLanes<R, Z>;
     constexpr int MB = S::MB, NW = S::NW, K = S::K, M = S::M, N = S::N, CB = S::CB;
     constexpr int UROW = S::UROW, OROW = S::OROW;
     __shared__ uint32_t smem[S::SMEM_WORDS];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const long long f0 = ((long long)blockIdx.x * S::WARPS + warp) * 32;
+    const long long f0 = ((long long)blockIdx.x * S::WARPS + warp) * per_warp;
     if (f0 >= frames) return;
-    const int nf = frames - f0 < 32 ? (int)(frames - f0) : 32;
-    uint32_t* const U = smem + warp * 32 * (UROW + OROW);
-    uint32_t* const O = U + 32 * UROW;
+    const int nf = frames - f0 < per_warp ? (int)(frames - f0) : per_warp;
+    uint32_t* const U = smem + warp * S::ROWS * (UROW + OROW);
+    uint32_t* const O = U + S::ROWS * UROW;
 
     /* A. pack the info bits of each frame (and copy the systematic bytes);
      * the loads of FA frames are issued before any is used, so that a warp
@@ -134,14 +146,14 @@ encode_lanes_kernel(const uint8_t* __restrict__ info, uint8_t* __restrict__ cw, 
                 uint32_t bits;
                 if constexpr (CB == 16) {
                     const uint4 w = v[a][r];
-                    if (q < KCH) reinterpret_cast<uint4*>(x)[q] = w;
+                    if (q < KCH) __stcs(reinterpret_cast<uint4*>(x) + q, w);
                     bits = nonzero_nibble(w.x) | (nonzero_nibble(w.y) << 4) | (nonzero_nibble(w.z) << 8) |
                            (nonzero_nibble(w.w) << 12);
                     bits |= __shfl_down_sync(0xffffffffu, bits, 1) << 16;
                     if (q < KCH && (q & 1) == 0) urow[q >> 1] = bits;
                 } else {
                     const uint2 w = v[a][r];
-                    if (q < KCH) reinterpret_cast<uint2*>(x)[q] = w;
+                    if (q < KCH) __stcs(reinterpret_cast<uint2*>(x) + q, w);
                     bits = nonzero_nibble(w.x) | (nonzero_nibble(w.y) << 4);
                     bits |= __shfl_down_sync(0xffffffffu, bits, 1) << 8;
                     bits |= __shfl_down_sync(0xffffffffu, bits, 2) << 16;
