@@ -434,7 +434,7 @@ int wldpc_syndrome_batch_host(wldpc_decoder* d, const int8_t* bits, int exit_ear
     return WLDPC_OK;
 }
 
-/* Host batch: chunks of kHostChunk frames rotate over kHostStages streams so
+/* Host batch: chunks of host_chunk() frames rotate over kHostStages streams so
  * that the copy-in of one chunk, the kernel of another and the copy-out of a
  * third overlap. post (nullable) receives the posterior; it may alias rx. */
 static int decode_host_pipeline(wldpc_decoder* d, const float* rx, float* post, int8_t* decoded,
@@ -443,7 +443,7 @@ static int decode_host_pipeline(wldpc_decoder* d, const float* rx, float* post, 
     if (!d || (frames && (!rx || !decoded))) return WLDPC_ERR_ARG;
     if (frames == 0) return WLDPC_OK;
     const size_t n = (size_t)d->code.n;
-    const size_t chunk = frames < kHostChunk ? frames : kHostChunk;
+    const size_t chunk = host_chunk(frames);
     int rc;
     for (int s = 0; s < kHostStages; s++) {
         if (!d->pipe[s]) CU(cudaStreamCreateWithFlags(&d->pipe[s], cudaStreamNonBlocking));

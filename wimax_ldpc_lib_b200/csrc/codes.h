@@ -31,13 +31,22 @@
 namespace wldpc {
 
 /* Host-buffer batch calls pipeline copy-in, decode and copy-out over
- * kHostStages streams in chunks of kHostChunk frames; with three stages chunk
- * k+2 is copied in while chunk k is copied out, so both copy directions stay
- * busy. (262,144 frames of rate 1/2 z = 96 on a B200, posterior back: 64.3 ms
- * with 8192-frame chunks, 65.8-66.2 with 16384, 64.7 with 4096; a fourth
- * stage did not help.) */
+ * kHostStages streams in chunks; with three stages chunk k+2 is copied in while
+ * chunk k is copied out, so both copy directions stay busy. A chunk is an
+ * eighth of the batch, between 1024 and 8192 frames: the last chunk's decode
+ * and copy out overlap with nothing (16,384 frames of rate 1/2 z = 96, hard
+ * bits back: 3.43 ms in chunks of 8192, 3.03 in chunks of 2048; the copy in
+ * alone takes 2.96), while large batches want long copies (262,144 frames,
+ * posterior back: 64.3 ms with 8192-frame chunks, 65.8-66.2 with 16384, 64.7
+ * with 4096; a fourth stage did not help). */
 constexpr int kHostStages = 3;
-constexpr unsigned long kHostChunk = 8192;
+constexpr unsigned long host_chunk(unsigned long frames)
+{
+    const unsigned long eighth = (frames + 7) / 8;
+    const unsigned long chunk = eighth < 1024 ? 1024 : eighth > 8192 ? 8192 : eighth;
+    return chunk < frames ? chunk : frames;
+}
+
 
 
 constexpr int kNB = 24;        /* base block columns */

@@ -382,7 +382,7 @@ static int lms_decode_host_pipeline(wldpc_lms* h, const float* rx, float* post, 
     if (!h || (frames && (!rx || !decoded))) return WLDPC_ERR_ARG;
     if (frames == 0) return WLDPC_OK;
     const size_t n = (size_t)h->code.n;
-    const size_t chunk = frames < kHostChunk ? frames : kHostChunk;
+    const size_t chunk = host_chunk(frames);
     int rc;
     for (int s = 0; s < kHostStages; s++) {
         if (!h->pipe[s]) CU(cudaStreamCreateWithFlags(&h->pipe[s], cudaStreamNonBlocking));
