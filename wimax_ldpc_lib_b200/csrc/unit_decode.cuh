@@ -9,7 +9,7 @@
  * its slowest frame stopped. Here a thread keeps its messages, one word per
  * non-zero block, in its own lane of TMEM (512 columns x 128 lanes = 256 KB
  * per SM, otherwise idle): 80 registers per thread, 24 warps on an SM (20 for
- * the 88 blocks of rate 3/4B). A layer's messages are loaded while the layer
+ * the 88 blocks of rate 3/4B, 16 for rate 5/6). A layer's messages are loaded while the layer
  * before runs (tcgen05.ld) and stored as they are made (tcgen05.st).
  *
  * One CTA per SM, all its warps cut into units: G frames (frame pairs for binary16) on UW = ceil(G z / 32)
@@ -72,7 +72,12 @@ struct UnitShape {
     static constexpr int G = unit_frames(Z, REFILL);
     static constexpr int ROWS = G * Z;               /* threads of a unit that own a row */
     static constexpr int UW = (ROWS + 31) / 32;      /* warps of a unit */
-    static constexpr int WARPS = 4 * (512 / NBLK);   /* as many as TMEM holds the messages of */
+    /* as many warps as TMEM holds the messages of; at degree 20 (rate 5/6) 16,
+     * whose 128 registers hold a row without spills (r5/6 z=60, 40,000 frames,
+     * 24 / 20 / 16 / 12 warps: plain 0.60 / 0.46 / 0.42 / 0.44 ms, learned 0.33 /
+     * 0.29 / 0.29 / 0.31), or 12 for plain units of three warps (z=96: 0.75 /
+     * 0.77 / 0.75 / 0.71: 15 warps load the SM's four schedulers unevenly) */
+    static constexpr int WARPS = R == 5 ? (REFILL && UW == 3 ? 12 : 16) : 4 * (512 / NBLK);
     static constexpr int U = UW == 1 ? WARPS : WARPS / UW < 15 ? WARPS / UW : 15;   /* 16 named barriers */
     static constexpr int THREADS = 32 * UW * U;
     static constexpr int SLOTS = U * G;

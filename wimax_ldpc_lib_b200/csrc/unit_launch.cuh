@@ -9,17 +9,16 @@ namespace wldpc {
 enum UnitKind : int { kUnitPlain = 0, kUnitLearned = 1, kUnitLearned16 = 2 };
 
 /* The smallest batch that goes to the unit kernel, per decoder, rate and z
- * (24 to 96 in steps of 4). A persistent CTA holds 16 to 24 frames (z = 32: 24,
- * z = 96: 8), so a small batch leaves most of it idle while each frame's
- * layers take longer than in a CTA of its own; a large batch gains by 24
- * warps per SM instead of 9 to 15 and by not waiting for a CTA's slowest
- * frame. All 114 codes were timed with both kernels at 64, 250, 600, 1200,
+ * (24 to 96 in steps of 4). A persistent CTA holds 4 to 32 frames or pairs (8 at
+ * r1/2 z = 96, 24 at z = 32), so a small batch leaves most of it idle while
+ * each frame's layers take longer than in a CTA of its own; a large batch gains
+ * by 16 to 24 warps per SM instead of 9 to 15 and by not waiting for a CTA's
+ * slowest frame. All 114 codes were timed with both kernels at 64, 250, 600, 1200,
  * 2500, 5000 and 30,000 frames (outputs identical); a code's line is the first
  * of those sizes from which on the unit kernel was never more than 1% slower.
  * Digits: 1: 64 frames, 2: 600, 3: 2500, 4: 5000, 5: 20,000, 0: never.
  * At 30,000 frames the unit kernel took, where it is used, 0.64-0.99 of the
- * other's time for plain (rate 5/6, degree 20, spills in 80 registers and
- * keeps the other kernel at most z), 0.55-0.99 for learned fp32 and 0.47-0.99
+ * other's time for plain, 0.55-0.99 for learned fp32 and 0.47-0.99
  * for binary16; least where z is no multiple of 16. */
 constexpr const char* kUnitMin[3][6] = {
     {
@@ -28,7 +27,7 @@ constexpr const char* kUnitMin[3][6] = {
         "5155335111511141114",
         "5153030131014141113",
         "5155440131013131110",
-        "0000000004030100500",
+        "5355510131314101115",
     },
     {
         "3151315111111151115",
@@ -36,7 +35,7 @@ constexpr const char* kUnitMin[3][6] = {
         "1113315311421331115",
         "1113530111112331215",
         "2111440111132231110",
-        "5154050344033342330",
+        "1253415112031241110",
     },
     {
         "1153415111511151114",
@@ -44,7 +43,7 @@ constexpr const char* kUnitMin[3][6] = {
         "1154315331533343115",
         "3154440333011343314",
         "2153310131033331113",
-        "5515550554044454540",
+        "3153315111431341114",
     },
 };
 constexpr long long unit_min_frames(UnitKind kind, int rate, int z)
