@@ -15,13 +15,13 @@ from test_learned16_gpu import random_weights
 pytestmark = pytest.mark.gpu
 
 # decoder, rate, z, frames
-CASES = [("plain", 0, 28, 64), ("plain", 0, 28, 63), ("plain", 0, 24, 20000), ("plain", 3, 36, 2501),
-         ("plain", 1, 44, 2500), ("plain", 0, 40, 5003), ("plain", 4, 60, 65), ("plain", 2, 52, 641),
-         ("plain", 0, 84, 333), ("plain", 0, 96, 2503), ("plain", 1, 64, 5000), ("plain", 5, 60, 2500),
-         ("learned", 1, 24, 64), ("learned", 2, 32, 67), ("learned", 5, 36, 2500), ("learned", 4, 44, 601),
-         ("learned", 3, 60, 300), ("learned", 0, 96, 600), ("learned", 5, 96, 2500), ("learned", 4, 68, 64),
-         ("half", 0, 24, 65), ("half", 1, 32, 2501), ("half", 3, 36, 5001), ("half", 4, 44, 64),
-         ("half", 5, 60, 2500), ("half", 0, 92, 129), ("half", 2, 96, 5001), ("half", 4, 84, 64)]
+CASES = [("plain", 0, 28, 64), ("plain", 0, 28, 63), ("plain", 1, 24, 15000), ("plain", 0, 36, 6001),
+         ("plain", 0, 44, 1800), ("plain", 0, 40, 6003), ("plain", 4, 60, 65), ("plain", 2, 52, 641),
+         ("plain", 0, 84, 333), ("plain", 1, 96, 6000), ("plain", 0, 64, 6000), ("plain", 5, 60, 2500),
+         ("learned", 1, 24, 1800), ("learned", 2, 32, 67), ("learned", 2, 36, 1801), ("learned", 5, 36, 6000),
+         ("learned", 4, 44, 6001), ("learned", 3, 60, 300), ("learned", 1, 96, 6000), ("learned", 4, 68, 1800),
+         ("half", 0, 24, 401), ("half", 0, 32, 6001), ("half", 0, 36, 6001), ("half", 2, 44, 6000),
+         ("half", 4, 28, 64), ("half", 5, 60, 2500), ("half", 0, 92, 129), ("half", 0, 96, 1801), ("half", 0, 84, 64)]
 
 
 def mixed_quality(oracle, rate, z, frames, seed):

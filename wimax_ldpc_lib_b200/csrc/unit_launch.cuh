@@ -13,42 +13,43 @@ enum UnitKind : int { kUnitPlain = 0, kUnitLearned = 1, kUnitLearned16 = 2 };
  * r1/2 z = 96, 24 at z = 32), so a small batch leaves most of it idle while
  * each frame's layers take longer than in a CTA of its own; a large batch gains
  * by 16 to 24 warps per SM instead of 9 to 15 and by not waiting for a CTA's
- * slowest frame. All 114 codes were timed with both kernels at 64, 250, 600, 1200,
- * 2500, 5000 and 30,000 frames (outputs identical); a code's line is the first
- * of those sizes from which on the unit kernel was never more than 1% slower.
- * Digits: 1: 64 frames, 2: 600, 3: 2500, 4: 5000, 5: 20,000, 0: never.
- * At 30,000 frames the unit kernel took, where it is used, 0.64-0.99 of the
- * other's time for plain, 0.55-0.99 for learned fp32 and 0.47-0.99
- * for binary16; least where z is no multiple of 16. */
+ * slowest frame. All 114 codes were timed with both kernels at eleven sizes
+ * from 64 to 30,000 frames, each at three Eb/N0 (outputs identical); a code's
+ * line is the first of the six below from which on the unit kernel was faster
+ * on the mean of the three, and at none of them more than 3.5% slower.
+ * Digits: 1: 64 frames, 2: 400, 3: 1800, 4: 6000, 5: 15,000, 6: 30,000, 0:
+ * never. At 30,000 frames the unit kernel took, where it is used, 0.64-0.99 of
+ * the other's time for plain, 0.55-0.99 for learned fp32 and 0.47-0.99 for
+ * binary16; least where z is no multiple of 16. */
 constexpr const char* kUnitMin[3][6] = {
     {
-        "5153435111212141113",
-        "5133535111014141113",
-        "5155335111511141114",
-        "5153030131014141113",
-        "5155440131013131110",
-        "5355510131314101115",
+        "6154436131413141114",
+        "5144535111033141114",
+        "5164535111513141114",
+        "6165045131014341114",
+        "5155540121034341110",
+        "6365616111445341115",
     },
     {
-        "3151315111111151115",
-        "4153510111013351113",
-        "1113315311421331115",
-        "1113530111112331215",
-        "2111440111132231110",
-        "1253415112031241110",
+        "2163516113511151115",
+        "3153530121033351114",
+        "1113535111533343115",
+        "1113430111333343335",
+        "1113440112133341310",
+        "5144555111033353110",
     },
     {
-        "1153415111511151114",
-        "1143335111533331113",
-        "1154315331533343115",
-        "3154440333011343314",
-        "2153310131033331113",
-        "3153315111431341114",
+        "2144445131533351113",
+        "1154445233634331113",
+        "4154445232633333334",
+        "4364445433013334445",
+        "6154440333033333315",
+        "5254316111543341114",
     },
 };
 constexpr long long unit_min_frames(UnitKind kind, int rate, int z)
 {
-    constexpr long long lines[6] = {-1, 64, 600, 2500, 5000, 20000};
+    constexpr long long lines[7] = {-1, 64, 400, 1800, 6000, 15000, 30000};
     return lines[kUnitMin[kind][rate][(z - 24) / 4] - '0'];
 }
 
