@@ -237,8 +237,7 @@ static int decode_launch(wldpc_decoder* d, const float* llr, int8_t* hard, float
     a.frames = (long long)frames;
     a.max_iter = (int)d->max_iter;
     a.wait_limit_us = d->wait_limit_us;
-    a.direct = direct;
-    return launch_tdmp(d->rate, d->z, d->mode, a, st) == cudaSuccess ? WLDPC_OK : WLDPC_ERR_CUDA;
+    return launch_tdmp(d->rate, d->z, d->mode, a, st, direct) == cudaSuccess ? WLDPC_OK : WLDPC_ERR_CUDA;
 }
 
 static int read_err(wldpc_decoder* d)

@@ -75,10 +75,11 @@ struct TdmpLaunch {
     int smem;           /* dynamic shared memory bytes (run-time z: 96 z) */
     bool runtime_z;     /* z, shifts and columns are passed in DecodeArgs */
     UnitLaunch<DecodeArgs> unit;   /* large batches, where it is the faster */
+    void (*direct)(const DecodeArgs);   /* LLRs in pinned host memory (single frames) */
 };
 /* entry for (rate, z, mode) or null if not built */
 const TdmpLaunch* tdmp_entry(int rate, int z, int mode);
-cudaError_t launch_tdmp(int rate, int z, int mode, const DecodeArgs& a, cudaStream_t st);
+cudaError_t launch_tdmp(int rate, int z, int mode, const DecodeArgs& a, cudaStream_t st, bool direct = false);
 
 }  // namespace wldpc
 

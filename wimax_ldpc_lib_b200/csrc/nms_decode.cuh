@@ -59,7 +59,6 @@ struct DecodeArgs {
     long long frames;
     int max_iter;
     unsigned wait_limit_us = kWaitLimitUs;   /* bound of the staging wait (the drain wait after a timeout is full) */
-    bool direct = false;    /* llr is pinned host memory: staged by ordinary loads, nothing to wait for */
     /* used only by the kernels whose z is a run-time value (ZT == 0): */
     int z;
     unsigned short shift[96];   /* per non-zero block, row-major over base rows */
@@ -312,7 +311,9 @@ __device__ __forceinline__ unsigned tdmp_rows_fail(At&& at)
     return fail;
 }
 
-template <int R, int ZT, int MODE>
+/* DIRECT: the LLRs are in pinned host memory and staged by ordinary loads, all
+ * in flight at once, with nothing to wait for (single frames) */
+template <int R, int ZT, int MODE, bool DIRECT = false>
 __global__ void __launch_bounds__(TdmpShape<R, ZT>::THREADS)
 tdmp_decode_kernel(const __grid_constant__ DecodeArgs a)
 {
@@ -344,15 +345,14 @@ tdmp_decode_kernel(const __grid_constant__ DecodeArgs a)
         s_last[1] = 0;
         s_half[0] = 0;
         s_half[1] = 0;
-        if (!a.direct) {
+        if constexpr (!DIRECT) {
             const uint32_t bytes = (uint32_t)(nf * N * 4);
             mbar_arrive_expect_tx(&bar, bytes);
             bulk_g2s(smem_post, a.llr + f0 * N, bytes, &bar);
         }
     }
     bool ok = a.wait_limit_us != 0;
-    if (a.direct) {
-        /* every load in flight at once: one trip over the bus */
+    if constexpr (DIRECT) {
         const float4* const src = reinterpret_cast<const float4*>(a.llr + f0 * N);
         float4 x[6];
 #pragma unroll
@@ -372,7 +372,7 @@ tdmp_decode_kernel(const __grid_constant__ DecodeArgs a)
     if (__syncthreads_or(!ok)) {
         if (tid == 0) {
             atomicOr(a.err, kErrWaitTimeout);
-            if (!a.direct) mbar_wait_bounded(&bar, 0, kWaitLimitUs);   /* let an in-flight copy land before exit */
+            if (!DIRECT) mbar_wait_bounded(&bar, 0, kWaitLimitUs);   /* let an in-flight copy land before exit */
         }
         return;
     }

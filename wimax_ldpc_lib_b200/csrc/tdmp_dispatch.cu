@@ -22,12 +22,12 @@ const TdmpLaunch* tdmp_entry(int rate, int z, int mode)
     return &kTdmpGeneric[rate][mode - 1];
 }
 
-cudaError_t launch_tdmp(int rate, int z, int mode, const DecodeArgs& args, cudaStream_t st)
+cudaError_t launch_tdmp(int rate, int z, int mode, const DecodeArgs& args, cudaStream_t st, bool direct)
 {
     const TdmpLaunch* e = tdmp_entry(rate, z, mode);
     if (!e) return cudaErrorInvalidValue;
     if (args.frames <= 0) return cudaSuccess;
-    if (!args.direct && unit_takes(e->unit, args.frames)) return launch_unit(e->unit, args, st);
+    if (!direct && unit_takes(e->unit, args.frames)) return launch_unit(e->unit, args, st);
     DecodeArgs a = args;
     int threads = e->threads, smem = e->smem;
     if (e->runtime_z) {
@@ -42,11 +42,12 @@ cudaError_t launch_tdmp(int rate, int z, int mode, const DecodeArgs& args, cudaS
     }
     const long long ctas = (a.frames + e->frames_per_cta - 1) / e->frames_per_cta;
     if (ctas > 0x7fffffffLL) return cudaErrorInvalidValue;
+    auto* const kernel = direct ? e->direct : e->kernel;
     if (smem > 48 * 1024) {
-        cudaError_t err = cudaFuncSetAttribute(e->kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (err != cudaSuccess) return err;
     }
-    e->kernel<<<(unsigned)ctas, threads, smem, st>>>(a);
+    kernel<<<(unsigned)ctas, threads, smem, st>>>(a);
     return cudaGetLastError();
 }
 

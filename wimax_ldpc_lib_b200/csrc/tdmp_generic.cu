@@ -5,7 +5,7 @@
 
 namespace wldpc {
 
-#define WLDPC_TDMP_GEN(R, M) {&tdmp_decode_kernel<R, 0, M>, 0, 1, 0, true, {}}
+#define WLDPC_TDMP_GEN(R, M) {&tdmp_decode_kernel<R, 0, M>, 0, 1, 0, true, {}, &tdmp_decode_kernel<R, 0, M, true>}
 
 extern const TdmpLaunch kTdmpGeneric[kRates][2] = {
     {WLDPC_TDMP_GEN(0, kOms), WLDPC_TDMP_GEN(0, kMs)}, {WLDPC_TDMP_GEN(1, kOms), WLDPC_TDMP_GEN(1, kMs)},

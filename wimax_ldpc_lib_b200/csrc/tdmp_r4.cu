@@ -7,7 +7,7 @@ namespace wldpc {
 
 #define WLDPC_TDMP_NMS(Z) \
     {&tdmp_decode_kernel<4, Z, kNms>, TdmpShape<4, Z>::THREADS, TdmpShape<4, Z>::G, TdmpShape<4, Z>::SMEM, false, \
-     unit_launch<4, Z, PlainRow>()}
+     unit_launch<4, Z, PlainRow>(), &tdmp_decode_kernel<4, Z, kNms, true>}
 
 extern const TdmpLaunch kTdmpNms_r4[kNumZ] = {
     WLDPC_TDMP_NMS(24), WLDPC_TDMP_NMS(28), WLDPC_TDMP_NMS(32), WLDPC_TDMP_NMS(36), WLDPC_TDMP_NMS(40),

@@ -26,9 +26,9 @@ constexpr const char* kUnitMin[3][6] = {
         "6154436131413141114",
         "5144535111033141114",
         "5164535111513141114",
-        "6165045131014341114",
+        "6165040131014341114",
         "5155540121034341110",
-        "6365616111445341115",
+        "6365610111445301115",
     },
     {
         "2163516113511151115",
@@ -42,7 +42,7 @@ constexpr const char* kUnitMin[3][6] = {
         "2144445131533351113",
         "1154445233634331113",
         "4154445232633333334",
-        "4364445433013334445",
+        "4364440433013334445",
         "6154440333033333315",
         "5254316111543341114",
     },
