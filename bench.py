@@ -329,8 +329,10 @@ def make_decoders(wl, rate, z, with_learned=True):
     return decs, meta
 
 
-KERNELS = {"plain": "tdmp_decode_kernel<{r},{z},NMS>", "learned": "lms_decode_kernel<{r},{z}>",
-           "learned_f16x2": "lms16_decode_kernel<{r},{z}>"}
+# the kernels that batches of this size go to; the fp32 learned decoder of rate 5/6 keeps one frame per CTA
+KERNELS = {"plain": "unit_decode_kernel<{r},{z},PlainRow>", "learned": "unit_decode_kernel<{r},{z},LearnedRow>",
+           "learned_f16x2": "unit_decode16_kernel<{r},{z}>"}
+C1_KERNELS = dict(KERNELS, learned="lms_decode_kernel<{r},{z}>")
 PROFILES = {"plain": "tdmp_nms_r{r}_z{z}.txt", "learned": "lms_r{r}_z{z}.txt", "learned_f16x2": "lms16_r{r}_z{z}.txt"}
 DTYPES = {"plain": "f32+f64", "learned": "f32", "learned_f16x2": "f16x2"}
 
@@ -524,7 +526,7 @@ def run_ours(args):
             r["hbm_frac"] = frames * 5 * n / (r["ms_per_step"] * 1e-3) / 1e9 / peak
             ir = issue_roofline(PROFILES[name].format(r=56, z=C1_Z), frames, r["ms_per_step"], clocks, sms)
             r["issue_frac"] = ir["frac"] if ir else None
-            r["kernel"] = KERNELS[name].format(r=C1_RATE, z=C1_Z)
+            r["kernel"] = C1_KERNELS[name].format(r=C1_RATE, z=C1_Z)
             c1[name] = r
             dec.close()
         extra["config1"] = {"workload": f"rate 5/6 z=96 (n=2304, k=1920), {frames} frames per GPU per step, "
