@@ -85,3 +85,23 @@ def test_unit_decoder_with_cap_zero_and_expired_waits(wl, cuda, oracle):
     dec.set_wait_limit(wl.WAIT_LIMIT_DEFAULT_US)
     check(cuda, dec, llr, reference(oracle, "plain", rate, z, 10, None, llr))
     dec.synchronize()
+
+
+@pytest.mark.parametrize("kind,scale", [("plain", None), ("learned", None), ("learned", 0.0), ("learned", -0.5),
+                                        ("half", None), ("half", 0.0)])
+def test_unit_decoders_on_infinite_llrs(wl, cuda, oracle, kind, scale):
+    """known bits as infinite LLRs: a third of them in every other frame, all in every third (with
+    a scale that is not positive their messages are 0, otherwise only frames without infinite errors)"""
+    rate, z, frames = 2, 52, 640
+    weights = None if kind == "plain" else random_weights(oracle, rate, z, 8, 9)[0]
+    if scale is not None:
+        weights[0] = scale
+    elif weights is not None:
+        weights[0] = np.abs(weights[0]) + np.float32(0.125)
+    llr = mixed_quality(oracle, rate, z, frames, 77)
+    n = llr.shape[1]
+    inf = np.float32(np.inf)
+    llr[::2, : n // 3] = np.where(llr[::2, : n // 3] > 0, inf, -inf)
+    rows = np.arange(0, frames, 3) if scale is not None else np.arange(3, frames, 4)
+    llr[rows] = np.where(llr[rows] > 0, inf, -inf)
+    check(cuda, handle(wl, kind, rate, z, 7, weights), llr, reference(oracle, kind, rate, z, 7, weights, llr))
