@@ -35,30 +35,49 @@ __global__ void mixed_count_kernel(const uint8_t* __restrict__ variant, const lo
     }
 }
 
-__global__ void mixed_plan_kernel(const int* __restrict__ counts, int* __restrict__ base, MixedItem* __restrict__ items,
-                                  int* __restrict__ num_items, int* __restrict__ queue, int chunk, long long per_rate)
+/* A block per rate: a warp scans the 19 counts, then all threads write the items. */
+constexpr int kPlanThreads = 256;
+__global__ void __launch_bounds__(kPlanThreads)
+mixed_plan_kernel(const int* __restrict__ counts, int* __restrict__ base, MixedItem* __restrict__ items,
+                  int* __restrict__ num_items, int* __restrict__ queue, int chunk, long long per_rate)
 {
-    const int rate = threadIdx.x;
-    if (blockIdx.x != 0 || rate >= kRates) return;
-    /* frame list: rates in order, z descending within a rate (long items first) */
-    int acc = 0;
-    for (int q = 0; q < rate; q++)
-        for (int zi = 0; zi < kNumZ; zi++) acc += counts[q * kNumZ + zi];
-    int k = 0;
-    MixedItem* it = items + (long long)rate * per_rate;
-    for (int zi = kNumZ - 1; zi >= 0; zi--) {
-        const int v = rate * kNumZ + zi;
-        base[v] = acc;
-        for (int s = 0; s < counts[v]; s += chunk) {
-            it[k].variant = v;
-            it[k].start = acc + s;
-            it[k].count = counts[v] - s < chunk ? counts[v] - s : chunk;
-            k++;
+    __shared__ int s_frame[kNumZ + 1], s_item[kNumZ + 1];   /* first frame and item of the j-th code */
+    const int rate = blockIdx.x, tid = threadIdx.x;
+    static_assert(kNumZ < 32, "a lane per code");
+    if (tid < 32) {
+        /* frame list: rates in order, z descending within a rate (long items first) */
+        int before = 0;
+        for (int v = tid; v < rate * kNumZ; v += 32) before += counts[v];
+        before = __reduce_add_sync(0xffffffffu, before);
+        const int v = rate * kNumZ + kNumZ - 1 - tid;
+        int frames = tid < kNumZ ? counts[v] : 0, n = (frames + chunk - 1) / chunk;
+        const int own = frames, own_n = n;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int f = __shfl_up_sync(0xffffffffu, frames, o), i = __shfl_up_sync(0xffffffffu, n, o);
+            if (tid >= o) {
+                frames += f;
+                n += i;
+            }
         }
-        acc += counts[v];
+        if (tid <= kNumZ) {   /* lane kNumZ has none of its own: the totals */
+            s_frame[tid] = before + frames - own;
+            s_item[tid] = n - own_n;
+        }
+        if (tid < kNumZ) base[v] = before + frames - own;
+        if (tid == kNumZ) {
+            num_items[rate] = n;
+            queue[rate] = 0;
+        }
     }
-    num_items[rate] = k;
-    queue[rate] = 0;
+    __syncthreads();
+    MixedItem* const it = items + (long long)rate * per_rate;
+    for (int j = 0; j < kNumZ; j++)
+        for (int k = s_item[j] + tid; k < s_item[j + 1]; k += kPlanThreads) {
+            const int start = s_frame[j] + (k - s_item[j]) * chunk, left = s_frame[j + 1] - start;
+            it[k].variant = rate * kNumZ + kNumZ - 1 - j;
+            it[k].start = start;
+            it[k].count = left < chunk ? left : chunk;
+        }
 }
 
 __global__ void mixed_scatter_kernel(const uint8_t* __restrict__ variant, const int* __restrict__ rank,
@@ -172,7 +191,7 @@ static int mixed_enqueue(wldpc_mixed* h, const uint8_t* variant, const long long
     if (cudaMemsetAsync(h->counts.p, 0, sizeof(int) * kVariants, st) != cudaSuccess) return WLDPC_ERR_CUDA;
     const unsigned gb = (unsigned)((nf + 255) / 256 < 4096 ? (nf + 255) / 256 : 4096);
     mixed_count_kernel<<<gb, 256, 0, st>>>(variant, offset, (int*)h->counts.p, (int*)h->rank.p, nf, h->err);
-    mixed_plan_kernel<<<1, 32, 0, st>>>((const int*)h->counts.p, (int*)h->base.p, (MixedItem*)h->items.p,
+    mixed_plan_kernel<<<kRates, kPlanThreads, 0, st>>>((const int*)h->counts.p, (int*)h->base.p, (MixedItem*)h->items.p,
                                        (int*)h->nitems.p, (int*)h->queue.p, chunk, per_rate);
     mixed_scatter_kernel<<<gb, 256, 0, st>>>(variant, (const int*)h->rank.p, (const int*)h->base.p,
                                             (int*)h->perm.p, nf);
