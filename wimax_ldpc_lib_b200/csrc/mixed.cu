@@ -35,7 +35,9 @@ __global__ void mixed_count_kernel(const uint8_t* __restrict__ variant, const lo
     }
 }
 
-/* A block per rate: a warp scans the 19 counts, then all threads write the items. */
+/* A block per rate: a warp scans the 19 counts, then all threads write the
+ * items (65,536 frames: 8 us, and the batch 3.06 -> 3.02 ms against one thread
+ * per rate that did all of it serially). */
 constexpr int kPlanThreads = 256;
 __global__ void __launch_bounds__(kPlanThreads)
 mixed_plan_kernel(const int* __restrict__ counts, int* __restrict__ base, MixedItem* __restrict__ items,
@@ -174,8 +176,10 @@ struct wldpc_mixed {
  * their slots more often and build the address table less often. Every chunk
  * of 1 to 24 frames and both CTA sizes timed on batches of all 114 codes (ms,
  * this choice against the 96 threads and 16 frames that it replaces): 256
- * frames 0.10 / 0.25, 1024 0.16 / 0.54, 4096 0.37 / 1.16, 16,384 0.95 / 2.63,
- * 65,536 3.06 / 5.44, 262,144 11.3 / 12.4. */
+ * frames 0.10 / 0.25, 1024 0.14 / 0.54, 4096 0.35 / 1.16, 16,384 0.91 / 2.63,
+ * 65,536 2.98 / 5.44, 262,144 11.1 / 12.4. The same number of frames for every
+ * z: with more where a CTA has more slots, the items of small z, the last ones,
+ * end less evenly (65,536 frames 3.15). */
 static void untuned_for(wldpc_mixed* h, size_t frames)
 {
     h->threads = 192;
