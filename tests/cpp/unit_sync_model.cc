@@ -73,9 +73,28 @@ static void votes()
     unit.any(true);
 }
 
+/* a unit that starts its next frames right after the last layer's stores */
+template <int R> static void clear()
+{
+    constexpr int NBLK = num_blocks(R), last = layer_degree(R, kMb[R] - 1);
+    uint32_t M[kMaxDeg] = {};
+    for (int a = 0; a < 512; a++) tm.column[a] = 1000u + a;
+    tm_ld<layer_degree(R, 0)>(M, 0);
+    for (int a = NBLK - last; a < NBLK; a++) store(a, 7u);
+    unit_clear_messages<R>(M, 0);
+    tm_wait_ld<layer_degree(R, 0)>(M);
+    tm_wait_st();
+    for (int a = 0; a < NBLK; a++)
+        if (tm.column[a]) std::printf("rate %d: message %d is %u\n", R, a, tm.column[a]), wrong++;
+    for (int e = 0; e < layer_degree(R, 0); e++)
+        if (M[e]) std::printf("rate %d: loaded message %d is %u\n", R, e, M[e]), wrong++;
+    if (tm.column[NBLK] != 1000u + NBLK) std::printf("rate %d: a column past the messages was stored\n", R), wrong++;
+}
+
 int main(int argc, char** argv)
 {
     if (argc == 2 && !std::strcmp(argv[1], "votes")) votes();
+    else if (argc == 2 && !std::strcmp(argv[1], "clear")) clear<0>(), clear<1>(), clear<2>(), clear<3>(), clear<4>(), clear<5>();
     else return 2;
     return wrong ? 1 : 0;
 }

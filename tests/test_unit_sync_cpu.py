@@ -16,7 +16,7 @@ def model(tmp_path_factory):
     return exe
 
 
-@pytest.mark.parametrize("what", ["votes"])
+@pytest.mark.parametrize("what", ["votes", "clear"])
 def test_nothing_out_of_order(model, what):
     r = subprocess.run([model, what], capture_output=True, text=True)
     assert r.returncode == 0, r.stdout

@@ -64,13 +64,16 @@ __device__ __forceinline__ uint32_t unit_tmem(uint32_t base, int warp, int nblk)
 {
     return base + ((uint32_t)(warp & 3) << 21) + (uint32_t)((warp >> 2) * nblk);
 }
-/* ... set to zero, and layer 0's loaded */
+/* ... set to zero, and layer 0's loaded. Nothing orders two stores to a column
+ * but a wait between them, so the last layer's, still in flight when a unit
+ * starts its next frames, are waited for first. */
 template <int R>
 __device__ __forceinline__ void unit_clear_messages(uint32_t (&M)[kMaxDeg], uint32_t tm)
 {
     constexpr int NBLK = num_blocks(R);
     const uint32_t zero[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     tm_wait_ld<layer_degree(R, 0)>(M);
+    tm_wait_st();
     static_for<(NBLK + 7) / 8>([&](auto C) {
         constexpr int c = 8 * decltype(C)::value;
         tm_st8(zero, tm + (c + 8 <= NBLK ? c : NBLK - 8));
