@@ -392,12 +392,31 @@ static inline float flip_sign(float x, unsigned neg)
     return v.f;
 }
 
+/* Inputs without NaN have the row's tracked minima; a NaN (inf - inf, or in the
+ * input) is no minimum of another edge and counts as positive in the row's
+ * sign, and an edge whose others are all NaN gets no message. Its hard bit is 0
+ * (x >= 0 is false), but the stopping rule counts it as 1 (x < 0 is false). */
+static float min_of_others(const float* L, int d, int e)
+{
+    float mu = NAN;
+    for (int q = 0; q < d; q++)
+        if (q != e) mu = fminf(mu, fabsf(L[q]));
+    return mu;
+}
+
+static unsigned learned_stops(const wo_code_t* c, const float* rx, int8_t* out)
+{
+    for (int v = 0; v < c->n; v++) out[v] = rx[v] < 0.0f ? 0 : 1;
+    const int stops = syndrome_one(c, out, 1) == 0;
+    slice(rx, out, c->n);
+    return stops;
+}
+
 static unsigned learned_one(const wo_code_t* c, int T, int cap, const float* A, const float* B, float* rx,
                             int8_t* out, float* msg, int32_t* iters, int32_t* synfail)
 {
     const int z = c->z;
-    slice(rx, out, c->n);
-    if (syndrome_one(c, out, 1) == 0) {
+    if (learned_stops(c, rx, out)) {
         if (iters) *iters = 0;
         if (synfail) *synfail = 0;
         return 0;
@@ -410,11 +429,15 @@ static unsigned learned_one(const wo_code_t* c, int T, int cap, const float* A, 
             for (int r = 0; r < z; r++) {
                 float L[WO_NB];
                 int v[WO_NB];
-                unsigned negpar = 0;
+                unsigned negpar = 0, nan = 0;
                 float m1 = INFINITY, m2 = INFINITY;
                 for (int e = 0; e < d; e++) {
                     v[e] = var_of(c, b0 + e, r);
                     L[e] = rx[v[e]] - msg[(b0 + e) * z + r];
+                    if (isnan(L[e])) {
+                        L[e] = NAN;
+                        nan = 1;
+                    }
                     negpar ^= (unsigned)(signbit(L[e]) != 0);
                     float a = fabsf(L[e]);
                     m2 = fminf(m2, fmaxf(m1, a));
@@ -424,7 +447,7 @@ static unsigned learned_one(const wo_code_t* c, int T, int cap, const float* A, 
                     unsigned neg_e = (unsigned)(signbit(L[e]) != 0);
                     /* positive LLR = bit 1: the extrinsic sign flips on odd-degree rows */
                     unsigned negmsg = negpar ^ neg_e ^ (unsigned)(d & 1);
-                    float mu = (fabsf(L[e]) == m1) ? m2 : m1;
+                    float mu = nan ? min_of_others(L, d, e) : (fabsf(L[e]) == m1) ? m2 : m1;
                     int col = c->blk_col[b0 + e];
                     float mag = fmaf(A[widx(t, i, col)], mu, -B[widx(t, i, col)]);
                     mag = fmaxf(mag, 0.0f);
@@ -434,8 +457,7 @@ static unsigned learned_one(const wo_code_t* c, int T, int cap, const float* A, 
                 }
             }
         }
-        slice(rx, out, c->n);
-        if (syndrome_one(c, out, 1) == 0) {
+        if (learned_stops(c, rx, out)) {
             if (iters) *iters = it + 1;
             if (synfail) *synfail = 0;
             return 0;

@@ -20,6 +20,9 @@
  * (a decoder may run past T with the weights of iteration T-1), and
  * the reference's stopping rule (slice x >= 0, stop at a zero syndrome).
  * Weights a = 0.815, b = 0 give a float normalized min-sum.
+ * A NaN L (from inf - inf, or in the input) is no minimum of another edge and
+ * counts as positive; an edge whose others are all NaN gets the message 0. The
+ * hard bit of a NaN is 0, though the stopping rule counts it as 1 (not x < 0).
  *
  * Messages: the decoder keeps every edge's message in a register of the
  * thread that owns the edge's row (one per non-zero block: 76 to 88), so

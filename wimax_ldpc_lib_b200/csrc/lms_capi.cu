@@ -5,7 +5,6 @@
  * offsets b, each [iteration][layer][base column]; entries of all-zero blocks
  * are ignored on input and returned as 0.
  */
-#include <cfloat>
 #include <cmath>
 #include <cstdint>
 #include <cstring>
@@ -313,18 +312,6 @@ static int lms16_launch_decode(wldpc_lms* h, const float* llr, int8_t* hard, flo
     return WLDPC_OK;
 }
 
-/* The unit kernel's relu is h + |h| of a halved product, NaN where fmaxf(h, 0)
- * is 0: under a scale that is not positive when the row's minimum is infinite
- * (LLRs of known bits). Tables with such a scale, or anything not finite, keep
- * the one-frame-per-CTA kernel; trained tables have none. */
-static bool lms_halvable(const wldpc_lms* h)
-{
-    for (int t = 0; t < h->T; t++)
-        for (int b = 0; b < h->nblk; b++)
-            if (!(h->w.a[t][b] >= 4 * FLT_MIN && h->w.a[t][b] <= FLT_MAX && fabsf(h->w.b[t][b]) <= FLT_MAX)) return false;
-    return true;
-}
-
 static int lms_launch_decode(wldpc_lms* h, const float* llr, int8_t* hard, float* post, int32_t* status,
                              size_t frames, cudaStream_t st)
 {
@@ -340,12 +327,10 @@ static int lms_launch_decode(wldpc_lms* h, const float* llr, int8_t* hard, float
     a.frames = (long long)frames;
     a.iters = h->cap;
     a.wrows = h->T;
-    const LmsLaunch* k = h->k;
-    const bool unit = unit_takes(k->unit, a.frames) && lms_halvable(h);
-    const float scale = unit ? 0.5f : 1.0f;   /* the unit kernel takes half the weights (LearnedRow) */
     for (int t = 0; t < h->T; t++)
-        for (int b = 0; b < h->nblk; b++) a.wab[t][b] = make_float2(h->w.a[t][b] * scale, h->w.b[t][b] * scale);
-    if (unit) {
+        for (int b = 0; b < h->nblk; b++) a.wab[t][b] = make_float2(h->w.a[t][b], h->w.b[t][b]);
+    const LmsLaunch* k = h->k;
+    if (unit_takes(k->unit, a.frames)) {
         CU(launch_unit(k->unit, a, st));
         return WLDPC_OK;
     }

@@ -12,7 +12,8 @@
  * compares and no selects.
  *
  * For values without NaN mu_e equals the tracked form's (|L_e| == min1 ?
- * min2 : min1), ties included. A NaN is never a minimum (fmin rule).
+ * min2 : min1), ties included. A NaN is never a minimum (fmin rule), unless
+ * an edge's others all are.
  */
 #ifndef WLDPC_MIN_OTHERS_CUH
 #define WLDPC_MIN_OTHERS_CUH

@@ -26,7 +26,7 @@
  *
  * Measured against the one-frame-per-CTA kernels of the same arithmetic (ms,
  * outputs identical): r1/2 z=96, 65,536 frames: plain 2.18 -> 2.05, learned
- * fp32 1.32 -> 1.29, binary16 (131,072) 1.66 -> 1.48; r2/3B z=44, 20,011
+ * fp32 1.32 -> 1.31, binary16 (131,072) 1.66 -> 1.48; r2/3B z=44, 20,011
  * frames: plain 0.326 -> 0.261, learned 0.26 -> 0.19; r3/4B z=28, 30,001
  * frames: 0.255 -> 0.193, 0.19 -> 0.14, binary16 0.17 -> 0.095. What binds
  * now: the ALU and XU pipes for plain (77% and 67% busy, 70% of the issue
@@ -89,10 +89,8 @@ struct UnitShape {
 
 /* ------------------------------------------------------ what a row does */
 
-/* learned min-sum in fp32 (lms.cuh). w: (a/2, b/2) of the iteration:
- * relu(a mu - b) is h + |h| with h = fma(a/2, mu, -b/2), an addition on the
- * FMA pipe in place of a maximum on the ALU pipe, which binds; halving is
- * exact except where |h| < 2^-126. */
+/* learned min-sum in fp32: the arithmetic of lms.cuh, so that a frame's outputs
+ * do not depend on the batch it comes in. w: (a, b) of the iteration. */
 struct LearnedRow {
     using Args = LmsArgs;
     static constexpr UnitKind kKind = kUnitLearned;
@@ -125,8 +123,7 @@ struct LearnedRow {
         const uint32_t one = ((sgn ^ ((uint32_t)(d & 1) << 31)) & 0x80000000u) | 0x3f800000u;
         static_for<d>([&](auto E) {
             const float2 ab = w[b0 + E];
-            const float h = __fmaf_rn(ab.x, mu[E], -ab.y);
-            const float mag = __fadd_rn(h, fabsf(h));
+            const float mag = fmaxf(__fmaf_rn(ab.x, mu[E], -ab.y), 0.0f);
             const float msg = __fmul_rn(mag, __uint_as_float((__float_as_uint(L[E]) & 0x80000000u) ^ one));
             m[E] = __float_as_uint(msg);
             pn[E] = __fadd_rn(L[E], msg);
