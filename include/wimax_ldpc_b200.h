@@ -361,9 +361,9 @@ WLDPC_API int wldpc_mixed_synchronize(wldpc_mixed* h);
  * concurrently or one after another. set_tuning and set_config leave the
  * rows per thread as they are; set_config / get_config also leave layout and
  * launch policy.
- * Until one of them or the autotuner is called, every decode sizes its work
- * items by its batch (192 threads; 1 to 16 frames), and get_tuning reports the
- * last choice. */
+ * Until set_tuning, set_config or the autotuner chooses them, every decode
+ * sizes its work items by its batch (192 threads; 1 to 16 frames), whatever
+ * the rows per thread, and get_tuning reports the last choice. */
 #define WLDPC_MIXED_MSG_REGISTERS 0
 #define WLDPC_MIXED_MSG_SHARED 1
 #define WLDPC_MIXED_CONCURRENT 0

@@ -146,7 +146,7 @@ static MixedKernel mixed_kernel(int ti, int layout, int rows, int rate)
 
 struct wldpc_mixed {
     unsigned max_iter;
-    bool tuned = false;                    /* the caller chose (or autotuned): untuned_for() does not */
+    bool tuned = false;                    /* threads and chunk are the caller's: untuned_for() leaves them */
     int threads = 96, layout = kMsgRegisters, chunk = 16;
     int rows = 1;                          /* expanded rows per thread: z / rows threads per frame */
     int launch = WLDPC_MIXED_CONCURRENT;   /* the six rate grids: concurrent or one after another */
@@ -370,8 +370,7 @@ int wldpc_mixed_get_tuning(wldpc_mixed* h, int* threads, int* layout, int* chunk
 int wldpc_mixed_set_rows_per_thread(wldpc_mixed* h, int rows)
 {
     if (!h || (rows != 1 && rows != 2)) return WLDPC_ERR_ARG;
-    h->tuned = true;
-    h->rows = rows;
+    h->rows = rows;   /* the work items stay sized by the batch, if they were */
     return WLDPC_OK;
 }
 
