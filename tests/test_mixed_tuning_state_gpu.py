@@ -36,3 +36,31 @@ def test_rows_per_thread_after_a_small_batch(wl, cuda, batches, rows):
     mixed.set_rows_per_thread(rows)
     holds_the_untuned_choice(cuda, mixed, batches)
     assert mixed.rows_per_thread() == rows
+
+
+@pytest.mark.parametrize("what", ["misaligned", "null", "bad code"])
+def test_an_autotune_that_fails_chooses_nothing(wl, cuda, batches, what):
+    mixed = wl.MixedDecoder(10)
+    variants, offsets, llr, hard = batches[300]
+    if what == "misaligned":
+        llr = llr[1:]
+    elif what == "null":
+        llr = None
+    else:
+        variants = variants.clone()
+        variants[7] = 114
+    with pytest.raises(wl.LdpcError) as e:
+        mixed.autotune(variants, offsets, llr, hard, repeats=1)
+    assert e.value.code == wl.ERR_ARG
+    holds_the_untuned_choice(cuda, mixed, batches)
+
+
+def test_an_autotune_that_fails_keeps_a_set_tuning(wl, cuda, batches):
+    mixed = wl.MixedDecoder(10)
+    mixed.set_tuning(96, wl.MIXED_MSG_SHARED, 3, wl.MIXED_SERIAL)
+    variants, offsets, llr, hard = batches[300]
+    with pytest.raises(wl.LdpcError):
+        mixed.autotune(variants, offsets, llr[1:], hard, repeats=1)
+    mixed.decode_device(*batches[300])
+    mixed.synchronize()
+    assert mixed.tuning() == (96, wl.MIXED_MSG_SHARED, 3, wl.MIXED_SERIAL)

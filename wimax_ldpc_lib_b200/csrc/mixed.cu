@@ -470,7 +470,6 @@ int wldpc_mixed_autotune(wldpc_mixed* h, const uint8_t* variant, const int64_t* 
                          int8_t* decoded, size_t frames, int repeats, float* best_ms)
 {
     if (!h || repeats < 1) return WLDPC_ERR_ARG;
-    h->tuned = true;
     static const int chunks[4] = {8, 16, 32, 64};
     float best = 1e30f;
     int bt = h->threads, bl = h->layout, bc = h->chunk, bp = h->launch, br = h->rows;
@@ -479,12 +478,20 @@ int wldpc_mixed_autotune(wldpc_mixed* h, const uint8_t* variant, const int64_t* 
         cudaGetLastError();
         return WLDPC_ERR_CUDA;
     }
-    auto restore = [&]() {
-        h->threads = bt;
-        h->layout = bl;
-        h->chunk = bc;
-        h->launch = bp;
-        h->rows = br;
+    const bool was_tuned = h->tuned;
+    h->tuned = true;   /* the candidates below stay as they are set; kept only if all of them ran */
+    auto use = [&](int threads, int layout, int chunk, int launch, int rows) {
+        h->threads = threads;
+        h->layout = layout;
+        h->chunk = chunk;
+        h->launch = launch;
+        h->rows = rows;
+    };
+    const int t0 = bt, l0 = bl, c0 = bc, p0 = bp, r0 = br;
+    auto fail = [&](int rc) {
+        use(t0, l0, c0, p0, r0);
+        h->tuned = was_tuned;
+        return rc;
     };
     /* CTA size x rows per thread x message layout x frames per work item x
      * launch policy, timed on the caller's batch */
@@ -493,11 +500,7 @@ int wldpc_mixed_autotune(wldpc_mixed* h, const uint8_t* variant, const int64_t* 
             for (int layout = 0; layout < 2; layout++)
                 for (int ci = 0; ci < 4; ci++)
                     for (int lp = 0; lp < 2; lp++) {
-                        h->threads = kThreadChoices[ti];
-                        h->rows = rows;
-                        h->layout = layout;
-                        h->chunk = chunks[ci];
-                        h->launch = lp;
+                        use(kThreadChoices[ti], layout, chunks[ci], lp, rows);
                         int rc = wldpc_mixed_decode_device(h, variant, offset, llr, decoded, nullptr, nullptr,
                                                            frames, h->stream);
                         if (!rc && cudaEventRecord(e0, h->stream) != cudaSuccess) rc = WLDPC_ERR_CUDA;
@@ -511,8 +514,7 @@ int wldpc_mixed_autotune(wldpc_mixed* h, const uint8_t* variant, const int64_t* 
                             cudaGetLastError();
                             cudaEventDestroy(e0);
                             cudaEventDestroy(e1);
-                            restore();
-                            return rc;
+                            return fail(rc);
                         }
                         float ms = 0.f;
                         cudaEventElapsedTime(&ms, e0, e1);
@@ -528,9 +530,10 @@ int wldpc_mixed_autotune(wldpc_mixed* h, const uint8_t* variant, const int64_t* 
                     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
-    restore();
+    use(bt, bl, bc, bp, br);
     if (best_ms) *best_ms = best;
-    return wldpc_mixed_synchronize(h);
+    const int rc = wldpc_mixed_synchronize(h);   /* a frame with a bad code or offset, or an expired wait */
+    return rc ? fail(rc) : WLDPC_OK;
 }
 
 }  // extern "C"
