@@ -377,7 +377,10 @@ WLDPC_API int wldpc_mixed_set_rows_per_thread(wldpc_mixed* h, int rows);
 WLDPC_API int wldpc_mixed_get_rows_per_thread(wldpc_mixed* h, int* rows);
 /* Times every (threads, rows per thread, layout, chunk, launch) candidate on
  * the given batch (repeats launches each) and keeps the fastest; *best_ms
- * (nullable) gets its time. */
+ * (nullable) gets its time. The chunks are 8, 16, 32 and 64 and the one that
+ * an untuned handle takes for this batch: if that is the fastest, decodes go
+ * on sizing their work items by the batch, with the rows, layout and launch
+ * policy found. A call that fails leaves the tuning as it was. */
 WLDPC_API int wldpc_mixed_autotune(wldpc_mixed* h, const uint8_t* variant, const int64_t* offset, const float* llr,
                                    int8_t* decoded, size_t frames, int repeats, float* best_ms);
 

@@ -64,3 +64,31 @@ def test_an_autotune_that_fails_keeps_a_set_tuning(wl, cuda, batches):
     mixed.decode_device(*batches[300])
     mixed.synchronize()
     assert mixed.tuning() == (96, wl.MIXED_MSG_SHARED, 3, wl.MIXED_SERIAL)
+
+
+def test_autotuning_a_small_batch_does_not_slow_it_down(wl, cuda, batches):
+    """300 frames of 114 codes need items of one frame, a chunk that the autotuner's
+    fixed ones (8 and more, twice the time) do not hold"""
+    def fastest(mixed):
+        times = []
+        for _ in range(20):
+            a, b = (cuda.cuda.Event(enable_timing=True) for _ in range(2))
+            a.record()
+            mixed.decode_device(*batches[300])
+            b.record()
+            b.synchronize()
+            times.append(a.elapsed_time(b))
+        return min(times)
+
+    untuned = fastest(wl.MixedDecoder(10))
+    mixed = wl.MixedDecoder(10)
+    mixed.autotune(*batches[300], repeats=5)
+    assert fastest(mixed) <= 1.3 * untuned
+    fixed = wl.MixedDecoder(10)
+    fixed.set_tuning(192, wl.MIXED_MSG_REGISTERS, 8)
+    assert fastest(fixed) > 1.3 * untuned   # or this test shows nothing
+    batches[13000][3].zero_()
+    mixed.decode_device(*batches[13000])
+    mixed.synchronize()
+    assert cuda.equal(batches[13000][3], batches["hard"])
+    assert mixed.tuning()[0::2] == batches["untuned"][0::2]

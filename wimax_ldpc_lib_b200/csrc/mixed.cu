@@ -493,6 +493,24 @@ int wldpc_mixed_autotune(wldpc_mixed* h, const uint8_t* variant, const int64_t* 
         h->tuned = was_tuned;
         return rc;
     };
+    /* times the tuning that use() set */
+    auto time_it = [&](float* ms) -> int {
+        int rc = wldpc_mixed_decode_device(h, variant, offset, llr, decoded, nullptr, nullptr, frames, h->stream);
+        if (!rc && cudaEventRecord(e0, h->stream) != cudaSuccess) rc = WLDPC_ERR_CUDA;
+        for (int k = 0; k < repeats && !rc; k++)
+            rc = wldpc_mixed_decode_device(h, variant, offset, llr, decoded, nullptr, nullptr, frames, h->stream);
+        if (!rc && (cudaEventRecord(e1, h->stream) != cudaSuccess || cudaEventSynchronize(e1) != cudaSuccess))
+            rc = WLDPC_ERR_CUDA;
+        if (!rc && cudaEventElapsedTime(ms, e0, e1) != cudaSuccess) rc = WLDPC_ERR_CUDA;
+        if (rc) {
+            cudaGetLastError();
+            cudaEventDestroy(e0);
+            cudaEventDestroy(e1);
+            return fail(rc);
+        }
+        *ms /= (float)repeats;
+        return WLDPC_OK;
+    };
     /* CTA size x rows per thread x message layout x frames per work item x
      * launch policy, timed on the caller's batch */
     for (int ti = 0; ti < 2; ti++)
@@ -501,24 +519,8 @@ int wldpc_mixed_autotune(wldpc_mixed* h, const uint8_t* variant, const int64_t* 
                 for (int ci = 0; ci < 4; ci++)
                     for (int lp = 0; lp < 2; lp++) {
                         use(kThreadChoices[ti], layout, chunks[ci], lp, rows);
-                        int rc = wldpc_mixed_decode_device(h, variant, offset, llr, decoded, nullptr, nullptr,
-                                                           frames, h->stream);
-                        if (!rc && cudaEventRecord(e0, h->stream) != cudaSuccess) rc = WLDPC_ERR_CUDA;
-                        for (int k = 0; k < repeats && !rc; k++)
-                            rc = wldpc_mixed_decode_device(h, variant, offset, llr, decoded, nullptr, nullptr,
-                                                           frames, h->stream);
-                        if (!rc && (cudaEventRecord(e1, h->stream) != cudaSuccess ||
-                                    cudaEventSynchronize(e1) != cudaSuccess))
-                            rc = WLDPC_ERR_CUDA;
-                        if (rc) {
-                            cudaGetLastError();
-                            cudaEventDestroy(e0);
-                            cudaEventDestroy(e1);
-                            return fail(rc);
-                        }
                         float ms = 0.f;
-                        cudaEventElapsedTime(&ms, e0, e1);
-                        ms /= repeats;
+                        if (const int rc = time_it(&ms)) return rc;
                         if (ms < best) {
                             best = ms;
                             bt = h->threads;
@@ -528,12 +530,35 @@ int wldpc_mixed_autotune(wldpc_mixed* h, const uint8_t* variant, const int64_t* 
                             br = h->rows;
                         }
                     }
+    /* ... and the work items that an untuned handle cuts this batch into, where
+     * none of the chunks above is as short (up to 45,000 frames): if they are
+     * the fastest, as they were from 100 to 16,384 frames (1024: 0.15 ms against
+     * 0.26 for the best fixed chunk), decodes go on sizing them by the batch */
+    bool sized = false;
+    untuned_for(h, frames);
+    const int ut = h->threads, uc = h->chunk;
+    if (uc < chunks[0])
+        for (int rows = 1; rows <= 2; rows++)
+            for (int layout = 0; layout < 2; layout++)
+                for (int lp = 0; lp < 2; lp++) {
+                    use(ut, layout, uc, lp, rows);
+                    float ms = 0.f;
+                    if (const int rc = time_it(&ms)) return rc;
+                    if (ms < best) {
+                        best = ms;
+                        bl = layout;
+                        bp = lp;
+                        br = rows;
+                        sized = true;
+                    }
+                }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
-    use(bt, bl, bc, bp, br);
     if (best_ms) *best_ms = best;
-    const int rc = wldpc_mixed_synchronize(h);   /* a frame with a bad code or offset, or an expired wait */
-    return rc ? fail(rc) : WLDPC_OK;
+    if (const int rc = wldpc_mixed_synchronize(h)) return fail(rc);   /* a bad code or offset, or an expired wait */
+    use(bt, bl, bc, bp, br);
+    h->tuned = !sized;
+    return WLDPC_OK;
 }
 
 }  // extern "C"
