@@ -52,6 +52,7 @@
 #ifndef WLDPC_LMS_CUH
 #define WLDPC_LMS_CUH
 
+#include <cfloat>
 #include <cstdint>
 #include "codes.h"
 #include "device_util.cuh"
@@ -529,6 +530,17 @@ lms_train_kernel(const __grid_constant__ LmsTrainArgs a)
                     if (e == i1) g_to_i2 += gmu;
                     else g_to_i1 += gmu;
                 });
+                /* a minimum that is infinite (known bits) times zero is NaN, but what relu
+                 * cut off, and an idle lane, adds nothing. By a branch of its own that few
+                 * rows take: a select per edge above took 4% of the step */
+                if (!(m2 <= FLT_MAX)) {
+                    static_for<d>([&](auto E_) {
+                        constexpr int e = decltype(E_)::value;
+                        const float2 ab = wab[b0 + e];
+                        const bool open = __fmaf_rn(ab.x, (fabsf(L[e]) == m1) ? m2 : m1, -ab.y) > 0.0f;
+                        if (!open || !owner) v[e / K][e % K] = 0.0f;
+                    });
+                }
                 static_for<d>([&](auto E_) {
                     constexpr int e = decltype(E_)::value;
                     const float sgn_l = __uint_as_float((__float_as_uint(L[e]) & 0x80000000u) | 0x3f800000u);
