@@ -248,6 +248,12 @@ WLDPC_API int wldpc_lms_set_precision(wldpc_lms* h, int precision);
 /* Decode on device buffers (layout and status as wldpc_decode_batch_device). */
 WLDPC_API int wldpc_lms_decode_device(wldpc_lms* h, const float* llr, int8_t* decoded, float* posterior,
                                       int32_t* status, size_t frames, void* stream);
+/* Waits for the device and reports a device-side error (WLDPC_ERR_TIMEOUT)
+ * recorded by earlier launches of this decoder, whose outputs are undefined. */
+WLDPC_API int wldpc_lms_synchronize(wldpc_lms* h);
+/* Test hook, as wldpc_decoder_set_wait_limit; batches that the binary16
+ * decoder stages without a copy have no wait and take no notice. */
+WLDPC_API int wldpc_lms_set_wait_limit(wldpc_lms* h, unsigned limit_us);
 /* Decode host buffers (posterior written back; num_errors = syndrome failed). */
 WLDPC_API int wldpc_lms_decode_host(wldpc_lms* h, float* rx_codewords, int8_t* decoded, uint32_t* num_errors,
                                     int32_t* status, size_t frames);

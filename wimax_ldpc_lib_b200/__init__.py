@@ -94,6 +94,8 @@ def _lib():
     L.wldpc_lms_set_weights.argtypes = [_p, _p]
     L.wldpc_lms_get_weights.argtypes = [_p, _p]
     L.wldpc_lms_decode_device.argtypes = [_p, _p, _p, _p, _p, _sz, _p]
+    L.wldpc_lms_synchronize.argtypes = [_p]
+    L.wldpc_lms_set_wait_limit.argtypes = [_p, _u]
     L.wldpc_lms_set_cap.argtypes = [_p, _u]
     L.wldpc_lms_set_precision.argtypes = [_p, _i]
     L.wldpc_lms_decode_host.argtypes = [_p, _p, _p, _p, _p, _sz]
@@ -467,6 +469,13 @@ class LearnedDecoder:
     def decode_device(self, llr, decoded, posterior=None, status=None, stream=None):
         _check(_lib().wldpc_lms_decode_device(self._h, _t_ptr(llr), _t_ptr(decoded), _t_ptr(posterior),
                                               _t_ptr(status), llr.shape[0], _stream_ptr(stream)), "lms decode")
+
+    def set_wait_limit(self, limit_us: int) -> None:
+        """Test hook: bound of the kernels' staging wait in microseconds (0 = time out at once)."""
+        _check(_lib().wldpc_lms_set_wait_limit(self._h, limit_us), "set_wait_limit")
+
+    def synchronize(self):
+        _check(_lib().wldpc_lms_synchronize(self._h), "synchronize")
 
     def decode_host(self, llr: np.ndarray):
         post = np.ascontiguousarray(llr, np.float32).copy()

@@ -136,6 +136,7 @@ struct wldpc_lms {
     bool host_stale = false; /* device weights changed by training */
     cudaStream_t stream = nullptr;
     unsigned* err = nullptr;
+    unsigned wait_limit_us = kWaitLimitUs;
     Buf wdev, mdev, vdev, grad, loss;                  /* training state: [2][T][nblk] */
     Buf ckp, ckm, gpart, lpart, tllr, tcw;             /* training scratch */
     Buf pllr[kHostStages], phard[kHostStages], pstat[kHostStages];                   /* host-batch pipeline staging */
@@ -169,6 +170,16 @@ static int lms_push_device_weights(wldpc_lms* h)
         }
     CU(cudaMemcpy(h->wdev.p, buf.data(), buf.size() * 4, cudaMemcpyHostToDevice));
     return WLDPC_OK;
+}
+
+/* reports and clears what earlier launches recorded */
+static int lms_read_err(wldpc_lms* h)
+{
+    unsigned e = 0;
+    CU(cudaMemcpy(&e, h->err, 4, cudaMemcpyDeviceToHost));
+    if (!e) return WLDPC_OK;
+    CU(cudaMemset(h->err, 0, 4));
+    return WLDPC_ERR_TIMEOUT;
 }
 
 extern "C" {
@@ -298,6 +309,7 @@ static int lms16_launch_decode(wldpc_lms* h, const float* llr, int8_t* hard, flo
     a.frames = (long long)frames;
     a.iters = h->cap;
     a.wrows = h->T;
+    a.wait_limit_us = h->wait_limit_us;
     for (int t = 0; t < h->T; t++)
         for (int b = 0; b < h->nblk; b++)
             a.wab[t][b] = make_uint2(half_pair_bits(h->w.a[t][b]), half_pair_bits(-h->w.b[t][b]));
@@ -327,6 +339,7 @@ static int lms_launch_decode(wldpc_lms* h, const float* llr, int8_t* hard, float
     a.frames = (long long)frames;
     a.iters = h->cap;
     a.wrows = h->T;
+    a.wait_limit_us = h->wait_limit_us;
     for (int t = 0; t < h->T; t++)
         for (int b = 0; b < h->nblk; b++) a.wab[t][b] = make_float2(h->w.a[t][b], h->w.b[t][b]);
     const LmsLaunch* k = h->k;
@@ -350,6 +363,20 @@ int wldpc_lms_decode_device(wldpc_lms* h, const float* llr, int8_t* decoded, flo
         return WLDPC_ERR_ARG;
     if (frames == 0) return WLDPC_OK;
     return lms_launch_decode(h, llr, decoded, posterior, status, frames, (cudaStream_t)stream);
+}
+
+int wldpc_lms_synchronize(wldpc_lms* h)
+{
+    if (!h) return WLDPC_ERR_ARG;
+    CU(cudaDeviceSynchronize());
+    return lms_read_err(h);
+}
+
+int wldpc_lms_set_wait_limit(wldpc_lms* h, unsigned limit_us)
+{
+    if (!h) return WLDPC_ERR_ARG;
+    h->wait_limit_us = limit_us;
+    return WLDPC_OK;
 }
 
 int wldpc_lms_set_precision(wldpc_lms* h, int precision)
@@ -421,12 +448,7 @@ static int lms_decode_host_pipeline(wldpc_lms* h, const float* rx, float* post, 
     }
     for (int s = 0; s < kHostStages; s++)
         if (cudaStreamSynchronize(h->pipe[s]) != cudaSuccess) return drain(WLDPC_ERR_CUDA);
-    unsigned e = 0;
-    CU(cudaMemcpy(&e, h->err, 4, cudaMemcpyDeviceToHost));
-    if (e) {
-        cudaMemset(h->err, 0, 4);
-        return WLDPC_ERR_TIMEOUT;
-    }
+    if ((rc = lms_read_err(h))) return rc;
     if (num_errors)
         for (size_t f = 0; f < frames; f++) num_errors[f] = (uint32_t)((st[f] >> 16) & 1);
     return WLDPC_OK;
