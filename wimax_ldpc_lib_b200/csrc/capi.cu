@@ -19,6 +19,7 @@
 
 #include "wimax_ldpc_b200.h"
 #include "codec_kernels.cuh"
+#include "host_batch.h"
 
 using namespace wldpc;
 
@@ -442,7 +443,9 @@ static int decode_host_pipeline(wldpc_decoder* d, const float* rx, float* post, 
     if (!d || (frames && (!rx || !decoded))) return WLDPC_ERR_ARG;
     if (frames == 0) return WLDPC_OK;
     const size_t n = (size_t)d->code.n;
-    const size_t chunk = host_chunk(frames);
+    /* statuses that only num_errors asks for go through a pageable vector */
+    const bool pinned = host_pinned(rx) && host_pinned(decoded) && host_pinned(status) && (status || !num_errors);
+    const size_t chunk = host_chunk(frames, n, pinned, post != nullptr);
     int rc;
     for (int s = 0; s < kHostStages; s++) {
         if (!d->pipe[s]) CU(cudaStreamCreateWithFlags(&d->pipe[s], cudaStreamNonBlocking));
