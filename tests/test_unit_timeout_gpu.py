@@ -14,7 +14,7 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("kind,rate,z,frames", [
     ("plain", 0, 44, 2000), ("plain", 1, 24, 15000), ("plain", 0, 84, 333), ("learned", 0, 28, 500),
-    ("learned", 4, 44, 6001), ("learned", 1, 96, 6000), ("half", 4, 28, 65), ("half", 0, 36, 6001), ("half", 0, 84, 65)])
+    ("learned", 4, 44, 6001), ("learned", 0, 52, 333), ("half", 4, 28, 401), ("half", 0, 36, 6001), ("half", 0, 84, 65)])
 def test_expired_waits_are_reported(wl, cuda, oracle, kind, rate, z, frames):
     weights = None if kind == "plain" else random_weights(oracle, rate, z, 8, 5)[0]
     llr = mixed_quality(oracle, rate, z, frames, 8)

@@ -14,37 +14,39 @@ enum UnitKind : int { kUnitPlain = 0, kUnitLearned = 1, kUnitLearned16 = 2 };
  * each frame's layers take longer than in a CTA of its own; a large batch gains
  * by 16 to 24 warps per SM instead of 9 to 15 and by not waiting for a CTA's
  * slowest frame. All 114 codes were timed with both kernels at eleven sizes
- * from 64 to 30,000 frames, each at three Eb/N0 (outputs identical); a code's
- * line is the first of the six below from which on the unit kernel was faster
- * on the mean of the three, and at none of them more than 3.5% slower.
+ * from 64 to 30,000 frames, each at three Eb/N0, launches back to back (outputs
+ * identical); from a code's line on, one of the six below, the unit kernel was
+ * faster on the mean of the three, and at none of them more than 3.5% slower (two
+ * runs differ by 2 to 4% at the small sizes). A change of either kernel wants
+ * them timed again.
  * Digits: 1: 64 frames, 2: 400, 3: 1800, 4: 6000, 5: 15,000, 6: 30,000, 0:
  * never. At 30,000 frames the unit kernel took, where it is used, 0.64-0.99 of
- * the other's time for plain, 0.55-0.99 for learned fp32 and 0.47-0.99 for
+ * the other's time for plain, 0.55-1.00 for learned fp32 and 0.47-0.99 for
  * binary16; least where z is no multiple of 16. */
 constexpr const char* kUnitMin[3][6] = {
     {
-        "6154436131413141114",
-        "5144535111033141114",
-        "5164535111513141114",
-        "6165040131014341114",
-        "5155540121034341110",
-        "6365610111445301115",
+        "6164436131413141114",
+        "5154535111033141114",
+        "5164535111514141114",
+        "6165040141014341314",
+        "6155540131034341110",
+        "6365610131445301115",
     },
     {
-        "2163516113511151115",
-        "3153530121033351114",
-        "1113535111533343115",
-        "1113430111333343335",
-        "1113440112133341310",
-        "5144555111033353110",
+        "5103516113031161115",
+        "5163530322033361135",
+        "5113536311533343315",
+        "5113430111333443335",
+        "4113440112133343330",
+        "5144556131033463110",
     },
     {
-        "2144445131533351113",
-        "1154445233634331113",
-        "4154445232633333334",
-        "4364440433013334445",
-        "6154440333033333315",
-        "5254316111543341114",
+        "2144445131533351114",
+        "1154445333634331114",
+        "4254445232633333335",
+        "6365450433013344445",
+        "6254440333033433316",
+        "5254346221543441115",
     },
 };
 constexpr long long unit_min_frames(UnitKind kind, int rate, int z)
