@@ -124,6 +124,17 @@ constexpr bool lms_index_addressing(int R, int Z)
     }
 }
 
+/* Codes whose schedule came out slower than with two tracked minima (4 to 15%
+ * for batches of 8 to 400 frames; all 114 timed), and what the compiler does
+ * better with there: the minima in two-input form (to the tracked form's time
+ * 0.94-1.00, rate 3/4B z = 32 0.73-0.79), or the layer's weights loaded ahead of
+ * the minima (0.73-0.92). Elsewhere the one or the other is slower by up to 20%. */
+constexpr bool lms_plain_minima(int R, int Z)
+{
+    return (R == 0 && Z == 28) || (R == 3 && Z == 32) || (R == 4 && (Z == 32 || Z == 40));
+}
+constexpr bool lms_early_weights(int R, int Z) { return Z == 64 && (R == 0 || R == 3 || R == 4); }
+
 template <int R, int Z, int I, int E>
 __device__ __forceinline__ float* lms_edge(float* P, float* Pr, float* Prz, int r)
 {
@@ -251,14 +262,18 @@ lms_decode_kernel(const __grid_constant__ LmsArgs a)
                     A[e] = fabsf(l);
                     sgn ^= __float_as_uint(l);   /* bit 31: parity of the negative L */
                 });
-                min_others<MinF32, d>(A, mu);
+                constexpr bool EARLY = lms_early_weights(R, Z);
+                float2 w[d];
+                if constexpr (EARLY) static_for<d>([&](auto E_) { w[E_] = wab[b0 + E_]; });
+                min_others<typename std::conditional<lms_plain_minima(R, Z), MinF32Plain, MinF32>::type, d>(A, mu);
                 /* positive LLR = bit 1: the extrinsic sign flips on odd-degree rows */
                 const uint32_t fb = (sgn ^ ((uint32_t)(d & 1) << 31)) & 0x80000000u;
                 const uint32_t fbo = fb | 0x3f800000u;   /* with sign(L_e): +-1.0 */
                 static_for<d>([&](auto E_) {
                     constexpr int e = decltype(E_)::value;
                     const float l = L[e];
-                    const float2 ab = wab[b0 + e];
+                    if constexpr (!EARLY) w[e] = wab[b0 + e];
+                    const float2 ab = w[e];
                     const float mag = fmaxf(__fmaf_rn(ab.x, mu[e], -ab.y), 0.0f);
                     const float msg = __fmul_rn(mag, __uint_as_float((__float_as_uint(l) & 0x80000000u) ^ fbo));
                     Mr[b0 + e] = msg;

@@ -35,6 +35,11 @@ struct MinF32 {
     }
 };
 
+/* ... the three-input minimum left to the compiler */
+struct MinF32Plain : MinF32 {
+    static __device__ __forceinline__ float min3(float a, float b, float c) { return fminf(fminf(a, b), c); }
+};
+
 /* two binary16 minima per word */
 struct MinH2 {
     using T = uint32_t;

@@ -36,8 +36,8 @@ constexpr const char* kUnitMin[3][6] = {
         "5103516113031161115",
         "5163530322033361135",
         "5113536311533343315",
-        "5113430111333443335",
-        "4113440112133343330",
+        "5123430111033443335",
+        "4153440112033343330",
         "5144556131033463110",
     },
     {
