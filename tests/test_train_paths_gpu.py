@@ -30,6 +30,7 @@ def test_a_message_cut_off_at_an_infinite_minimum_has_no_gradient(wl, cuda, orac
     T = 8
     w, rs, cols = random_weights(oracle, rate, z, T, 11)
     w[0, :, 0] = scale
+    w[1, 1::2, 0] *= -1   # offsets of both signs
     _, cw, llr = inputs.frames(oracle, rate, z, 24, 1.75, seed=90)
     for c in cols[:rs[1]]:
         known = slice(c * z, (c + 1) * z)

@@ -46,6 +46,7 @@
  * Subgradients: sign() and the argmin choice are constant, d|x|/dx = sign(x),
  * relu'(0) = 0; edge e != i1 takes its magnitude from i1 (the first edge with
  * |L| == min1), edge i1 from i2 (the first other edge with |L| == min2).
+ * An infinite minimum (known bits) counts as the largest finite number.
  * A CTA adds up the weight gradients of its frames; a second kernel adds the
  * CTAs' in a fixed order (deterministic) and applies Adam.
  */
@@ -415,7 +416,7 @@ __device__ __forceinline__ float warp_sums(float (&v)[K], int lane)
  * the backward pass reads, only the message gradients stay in shared memory,
  * the rows' weight gradients are summed over a warp 16 or 32 at a time, and a
  * CTA adds its frames' gradients up (fixed order) instead of writing each:
- * a step of 4096 r1/2 z=96 frames 6.07 -> 1.81 ms.
+ * a step of 4096 r1/2 z=96 frames 6.07 -> 1.83 ms.
  * The last iteration is run once: its L are recorded on the way forward. */
 template <int R, int Z>
 __global__ void __launch_bounds__(LmsTrainShape<R, Z>::THREADS, LmsTrainShape<R, Z>::MIN_CTAS)
@@ -458,7 +459,12 @@ lms_train_kernel(const __grid_constant__ LmsTrainArgs a)
 #pragma unroll
         for (int q = 0; q < NBLK; q++) m[q] = 0.0f;
         auto weights = [&](int t) {   /* between two barriers */
-            for (int q = tid; q < NBLK; q += TH) wab[q] = make_float2(a.wa[t * NBLK + q], a.wb[t * NBLK + q]);
+            for (int q = tid; q < NBLK; q += TH) {
+                const float2 ab = make_float2(a.wa[t * NBLK + q], a.wb[t * NBLK + q]);
+                /* a scale of 0 makes no message of an infinite minimum, whatever the offset: a
+                 * hair below 0, which no finite minimum feels, says so of the largest one too */
+                wab[q] = make_float2(ab.x == 0.0f ? -1e-30f : ab.x, ab.y);
+            }
         };
 
         /* forward, keeping what each iteration ends with except the last two:
@@ -521,6 +527,12 @@ lms_train_kernel(const __grid_constant__ LmsTrainArgs a)
                     constexpr int e = d - 1 - decltype(E_)::value;
                     i2 = fabsf(L[e]) == m2 && e != i1 ? e : i2;
                 });
+                /* an infinite minimum (known bits) as the largest finite one: times zero it
+                 * is NaN, but what relu cut off, and an idle lane, adds nothing. (Cleared
+                 * edge by edge instead, by selects or behind a branch that few rows take:
+                 * 4% slower at r1/2 z=96, 4-20% at the other rates.) */
+                m1 = fminf(m1, FLT_MAX);
+                m2 = fminf(m2, FLT_MAX);
                 constexpr int K = 2 * d <= 16 ? 16 : 32;
                 constexpr int H = (2 * d + K - 1) / K;    /* groups of K sums (2 for d = 20) */
                 float v[H][K];
@@ -545,17 +557,6 @@ lms_train_kernel(const __grid_constant__ LmsTrainArgs a)
                     if (e == i1) g_to_i2 += gmu;
                     else g_to_i1 += gmu;
                 });
-                /* a minimum that is infinite (known bits) times zero is NaN, but what relu
-                 * cut off, and an idle lane, adds nothing. By a branch of its own that few
-                 * rows take: a select per edge above took 4% of the step */
-                if (!(m2 <= FLT_MAX)) {
-                    static_for<d>([&](auto E_) {
-                        constexpr int e = decltype(E_)::value;
-                        const float2 ab = wab[b0 + e];
-                        const bool open = __fmaf_rn(ab.x, (fabsf(L[e]) == m1) ? m2 : m1, -ab.y) > 0.0f;
-                        if (!open || !owner) v[e / K][e % K] = 0.0f;
-                    });
-                }
                 static_for<d>([&](auto E_) {
                     constexpr int e = decltype(E_)::value;
                     const float sgn_l = __uint_as_float((__float_as_uint(L[e]) & 0x80000000u) | 0x3f800000u);
