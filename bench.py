@@ -329,10 +329,20 @@ def make_decoders(wl, rate, z, with_learned=True):
     return decs, meta
 
 
-# the kernels that batches of this size go to; the fp32 learned decoder of rate 5/6 keeps one frame per CTA
-KERNELS = {"plain": "unit_decode_kernel<{r},{z},PlainRow>", "learned": "unit_decode_kernel<{r},{z},LearnedRow>",
-           "learned_f16x2": "unit_decode16_kernel<{r},{z}>"}
-C1_KERNELS = dict(KERNELS, learned="lms_decode_kernel<{r},{z}>")
+# from 30,000 frames on, the highest line of any code, batches go to the large-batch kernels; the fp32
+# learned decoder of rate 5/6 has none at z = 96
+KERNELS = {"plain": ("tdmp_decode_kernel<{r},{z},NMS>", "unit_decode_kernel<{r},{z},PlainRow>"),
+           "learned": ("lms_decode_kernel<{r},{z}>", "unit_decode_kernel<{r},{z},LearnedRow>"),
+           "learned_f16x2": ("lms16_decode_kernel<{r},{z}>", "unit_decode16_kernel<{r},{z}>")}
+
+
+def kernel_name(decoder, rate, z, frames):
+    small, large = (k.format(r=rate, z=z) for k in KERNELS[decoder])
+    if decoder == "learned" and rate == 5:
+        return small
+    return large if frames >= 30000 else f"{small} or {large}, by the batch size"
+
+
 PROFILES = {"plain": "tdmp_nms_r{r}_z{z}.txt", "learned": "lms_r{r}_z{z}.txt", "learned_f16x2": "lms16_r{r}_z{z}.txt"}
 DTYPES = {"plain": "f32+f64", "learned": "f32", "learned_f16x2": "f16x2"}
 
@@ -494,7 +504,7 @@ def run_ours(args):
     prof = PROFILES[head].format(r=12, z=Z)
     roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                 "traffic": load_profile_value(prof, "traffic_bytes_per_launch_full_batch"), "peak_kind": peak_kind,
-                "kernel": KERNELS[head].format(r=RATE, z=Z), "algorithmic_bytes_per_launch": bytes_per_launch,
+                "kernel": kernel_name(head, RATE, Z, frames), "algorithmic_bytes_per_launch": bytes_per_launch,
                 "note": "5n bytes per frame (float32 LLR read + int8 hard-decision write); the decoders are "
                         "instruction-issue bound, not HBM-bound: see the issue roofline"}
     iss = issue_roofline(prof, frames, ms, clocks, sms)
@@ -526,7 +536,7 @@ def run_ours(args):
             r["hbm_frac"] = frames * 5 * n / (r["ms_per_step"] * 1e-3) / 1e9 / peak
             ir = issue_roofline(PROFILES[name].format(r=56, z=C1_Z), frames, r["ms_per_step"], clocks, sms)
             r["issue_frac"] = ir["frac"] if ir else None
-            r["kernel"] = C1_KERNELS[name].format(r=C1_RATE, z=C1_Z)
+            r["kernel"] = kernel_name(name, C1_RATE, C1_Z, frames)
             c1[name] = r
             dec.close()
         extra["config1"] = {"workload": f"rate 5/6 z=96 (n=2304, k=1920), {frames} frames per GPU per step, "

@@ -379,7 +379,7 @@ const EncLanesLaunch* enc_lanes_entry(int rate, int z)
 }
 
 /* Frames per warp of the lane-per-frame encoder: 4, whose loads are all issued
- * at once, or 8, which spread phase B's fixed work over more of them, where
+ * at once (three, then one, where a frame has more than 96 chunks), or 8, which spread phase B's fixed work over more of them, where
  * frames are short and the batch fills the GPU with 8 (148 SMs x 4 warps).
  * Timed at 2 to 32 per warp, seven codes, 600 to 262,144 frames (us, 4 / 8):
  * z=96 141 / 148, z=64 96 / 100, z=60 113 / 119, z=48 82 / 76, z=24 52 / 45 at

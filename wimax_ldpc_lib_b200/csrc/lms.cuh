@@ -335,7 +335,8 @@ struct LmsTrainArgs {
 __device__ __forceinline__ float softplus_f(float x) { return x > 0.0f ? x + log1pf(__expf(-x)) : log1pf(__expf(x)); }
 __device__ __forceinline__ float sigmoid_f(float x) { return 1.0f / (1.0f + __expf(-x)); }
 
-/* One frame at a time per CTA of whole warps (lanes past z idle along). */
+/* One frame at a time per CTA of whole warps. Lanes past z idle along on another
+ * lane's row: what they read, maybe while it is written, reaches no sum. */
 template <int R, int Z>
 struct LmsTrainShape {
     static constexpr int MB = kMb[R];

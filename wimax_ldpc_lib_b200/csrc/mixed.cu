@@ -176,8 +176,8 @@ struct wldpc_mixed {
  * their slots more often and build the address table less often. Every chunk
  * of 1 to 24 frames and both CTA sizes timed on batches of all 114 codes (ms,
  * this choice against the 96 threads and 16 frames that it replaces): 256
- * frames 0.10 / 0.25, 1024 0.14 / 0.54, 4096 0.35 / 1.16, 16,384 0.91 / 2.63,
- * 65,536 2.98 / 5.44, 262,144 11.1 / 12.4. The same number of frames for every
+ * frames 0.09 / 0.25, 1024 0.15 / 0.54, 4096 0.35 / 1.06, 16,384 0.91 / 2.77,
+ * 65,536 2.98 / 5.24, 262,144 11.1 / 12.1. The same number of frames for every
  * z: with more where a CTA has more slots, the items of small z, the last ones,
  * end less evenly (65,536 frames 3.15). */
 static void untuned_for(wldpc_mixed* h, size_t frames)

@@ -77,7 +77,9 @@ struct UnitShape {
      * whose 128 registers hold a row without spills (r5/6 z=60, 40,000 frames,
      * 24 / 20 / 16 / 12 warps: plain 0.60 / 0.46 / 0.42 / 0.44 ms, learned 0.33 /
      * 0.29 / 0.29 / 0.31), or 12 for plain units of three warps (z=96: 0.75 /
-     * 0.77 / 0.75 / 0.71: 15 warps load the SM's four schedulers unevenly) */
+     * 0.77 / 0.75 / 0.71: 15 warps load the SM's four schedulers unevenly). Rows of
+     * degree 10 to 15 spill too in 80 or 96 registers, plain rate 3/4A most (124 to
+     * 328 bytes per thread); fewer warps were not timed there. */
     static constexpr int WARPS = R == 5 ? (REFILL && UW == 3 ? 12 : 16) : 4 * (512 / NBLK);
     static constexpr int U = UW == 1 ? WARPS : WARPS / UW < 15 ? WARPS / UW : 15;   /* 16 named barriers */
     static constexpr int THREADS = 32 * UW * U;
@@ -194,7 +196,9 @@ unit_decode_kernel(const __grid_constant__ typename Row::Args a)
     const int tid = threadIdx.x, warp = tid >> 5;
     const int u = S::UW == 1 ? warp : tid / UT;
     const int q = tid - u * UT;
-    const bool owner = FULL || q < S::ROWS;   /* the other lanes compute along and store nothing */
+    /* the other lanes compute along and store nothing: what they read, maybe while
+     * its row's owner writes it, reaches no posterior, vote or output */
+    const bool owner = FULL || q < S::ROWS;
     const int g = G == 1 || !owner ? 0 : q / Z;
     const int r = owner ? q - g * Z : (q - S::ROWS) % Z;
     const int slot = u * G + g;

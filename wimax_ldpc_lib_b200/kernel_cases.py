@@ -4,10 +4,12 @@ for profilers (ncu: every launch below is one capture) and quick timing.
   python -m wimax_ldpc_lib_b200.kernel_cases [--frames F] [--cases decode,encode,train,syndrome,bits,lfsr,nullspace]
 
   decode     F frames of rate 1/2 z = 96 at 2.25 dB and of rate 5/6 z = 96 at
-             4 dB (framegen_kernel), each decoded once by the plain decoder
-             (tdmp_decode_kernel), the learned decoder with its shipped
-             weights (lms_decode_kernel) and the same weights in packed
-             binary16 (lms16_decode_kernel), cap 10
+             4 dB (framegen_kernel), each decoded once by the plain decoder,
+             the learned decoder with its shipped weights and the same weights
+             in packed binary16, cap 10: by unit_decode_kernel and
+             unit_decode16_kernel from each code's line on (unit_launch.cuh),
+             below it, and where a code has none (fp32 learned, rate 5/6),
+             by tdmp_decode_kernel, lms_decode_kernel and lms16_decode_kernel
   encode     F rate 1/2 z = 96 info words (encode_lanes_kernel)
 
   train      one Adam step of the learned decoder's training (rate 1/2,
